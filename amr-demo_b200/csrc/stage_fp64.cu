@@ -15,17 +15,11 @@ namespace amrgpu {
 
 struct FluxOpsFP64 {
     __device__ static __forceinline__ void prims(const double *q, double *P) { cell_prims_fp64(q, P); }
-    __device__ static __forceinline__ void roe(const double *l, const double *r, double n0, double n1,
-                                               double *f)
+    // the lanes of a warp mix x- and y-faces here, so the direction is a
+    // select and not a branch into one copy per direction
+    __device__ static __forceinline__ void roe(const double *l, const double *r, double n0, double n1, double *f)
     {
-        roe_flux_prim_fp64(l, r, n0, n1, f);
-    }
-    // the exact form evaluates every face through the general expression
-    template <int DIR>
-    __device__ static __forceinline__ void roe_axis(const double *l, const double *r, double n0, double n1,
-                                                    double *f)
-    {
-        roe_flux_prim_fp64(l, r, n0, n1, f);
+        roe_flux_prim_fp64<2>(l, r, n0, n1, f);
     }
     __device__ static __forceinline__ void bc(int bc, const double *q, double n0, double n1,
                                               const double *qin, double *f)
@@ -36,6 +30,7 @@ struct FluxOpsFP64 {
     {
         return cfl_candidate_fp64(q, vol, c);
     }
+    __device__ static __forceinline__ void rate(const double *r, double vol, double *k) { residual_rate(r, vol, k); }
 };
 
 // solver_time_step_2d_module.F90:26-122 over every cell, folded with the
@@ -142,15 +137,15 @@ const void *cfl_kernel_fp64(int n)
 // way to the size's first block kernel on meshes too small to fill the GPU
 // with sweep warps); the autotuner picks among all entries of the size.
 static const StageLaunch kTable64[] = {
+    AMRGPU_SWEEP64_16(4, 3),  // 168 registers, 12 warps per SM
     AMRGPU_SWEEP64_16(4, 4),  // 128 registers, 16 warps per SM
     AMRGPU_SWEEP64_16(2, 8),
-    AMRGPU_SWEEP64_16(4, 3),
     AMRGPU_STAGE64(16, 1, 288, 2),
     AMRGPU_STAGE64(16, 1, 288, 1),
     AMRGPU_STAGE64(16, 2, 576, 1),
     AMRGPU_STAGE64(16, 1, 256, 2),
-    AMRGPU_SWEEP64_8(4, 4),   // two 8x8 quads per warp
-    AMRGPU_SWEEP64_8(4, 3),
+    AMRGPU_SWEEP64_8(4, 3),   // two 8x8 quads per warp
+    AMRGPU_SWEEP64_8(4, 4),
     AMRGPU_STAGE64(8, 4, 288, 2),
     AMRGPU_STAGE64(8, 2, 160, 3),
     AMRGPU_STAGE64(8, 4, 576, 1),

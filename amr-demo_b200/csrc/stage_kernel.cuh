@@ -148,13 +148,19 @@ __device__ __forceinline__ double cell_h_of(double h_base, int level, int n)
 }
 
 // Volume of the sub-cell with nodes n1..n4:
-// 0.5*sqrt(((n4-n1) x (n3-n2))**2), solver_residual_subgrid_2d_module.F90:152-160
+// 0.5*sqrt(((n4-n1) x (n3-n2))**2), solver_residual_subgrid_2d_module.F90:152-160.
+// The root of a rounded square is the absolute value itself in binary
+// round-to-nearest when the square neither over- nor underflows (S. Boldo,
+// "Stupid is as stupid does: taking the square root of the square of a
+// floating-point number", 2015), so the root is only taken outside that range.
 __device__ __forceinline__ double subcell_volume(double x1, double y1, double x2, double y2,
                                                  double x3, double y3, double x4, double y4)
 {
     double v1x = x4 - x1, v1y = y4 - y1;
     double v2x = x3 - x2, v2y = y3 - y2;
     double cr = v1x * v2y - v1y * v2x;
+    const double mag = fabs(cr);
+    if (mag >= 0x1p-500 && mag <= 0x1p500) return 0.5 * mag;
     return 0.5 * sqrt(cr * cr);
 }
 
@@ -734,7 +740,8 @@ __global__ void __launch_bounds__(T, MINB) stage_kernel(const StageArgs a)
             load_rec<F32>(pq, li, Lp);
             load_rec<F32>(pq, ri, Rp);
             if (bcv < 0) {
-                if (xd) FluxOps::template roe_axis<0>(Lp, Rp, n0, n1, fl);
+                if constexpr (!F32) FluxOps::roe(Lp, Rp, n0, n1, fl);
+                else if (xd) FluxOps::template roe_axis<0>(Lp, Rp, n0, n1, fl);
                 else FluxOps::template roe_axis<1>(Lp, Rp, n0, n1, fl);
             } else {
                 R qin[4] = {(R)a.qinflow[0], (R)a.qinflow[1], (R)a.qinflow[2], (R)a.qinflow[3]};
@@ -775,7 +782,8 @@ __global__ void __launch_bounds__(T, MINB) stage_kernel(const StageArgs a)
                 alignas(16) R fl[4];
                 load_rec<F32>(pq, (s & 1) ? own : nb, Lp);
                 load_rec<F32>(pq, (s & 1) ? nb : own, Rp);
-                if (xd) FluxOps::template roe_axis<0>(Lp, Rp, h, (R)0, fl);
+                if constexpr (!F32) FluxOps::roe(Lp, Rp, xd ? h : (R)0, xd ? (R)0 : h, fl);
+                else if (xd) FluxOps::template roe_axis<0>(Lp, Rp, h, (R)0, fl);
                 else FluxOps::template roe_axis<1>(Lp, Rp, (R)0, h, fl);
                 store_flux<F32>(fh, (ql * 4 + s) * N + m, fl);
             }
@@ -867,7 +875,7 @@ __global__ void __launch_bounds__(T, MINB) stage_kernel(const StageArgs a)
             }
             double vol;
             double kv[4];
-            if (F32) {
+            if constexpr (F32) {
                 vol = geo[8 * ql + 3];
                 const double inv = geo[8 * ql + 2];
 #pragma unroll
@@ -877,8 +885,7 @@ __global__ void __launch_bounds__(T, MINB) stage_kernel(const StageArgs a)
                 const double *n1p = nd + 2 * (j * NP1 + i);
                 const double *n3p = nd + 2 * ((j + 1) * NP1 + i);
                 vol = subcell_volume(n1p[0], n1p[1], n1p[2], n1p[3], n3p[0], n3p[1], n3p[2], n3p[3]);
-#pragma unroll
-                for (int f = 0; f < 4; ++f) kv[f] = (r[f] / vol) * -1.0;
+                FluxOps::rate(r, vol, kv);
             }
 
             const long long gi = (long long)(q0 + ql) * NN + c;

@@ -22,19 +22,29 @@
 //           2/3; a coarse hanging edge also its second, index-paired flux)
 //           into a per-warp table, and the faces between rows R-1 and R;
 //   sweep   at step t lane (i, h) takes cell (i, j = Rh+t): its record, the
-//           bilinear nodes of row j+1 at columns i and i+1 (row j's came
-//           from the step before), then two flux evaluations through one
-//           call site -- the x-face at i-1/2 with the left neighbour's record
-//           taken by a warp shuffle (its value goes to lane i-1, which needs
-//           it as its i+1/2 face, by a second shuffle), then the y-face at
-//           j-1/2 with the record of row j-1, which completes row j-1 (its
-//           update is written).
+//           y-face flux at j-1/2 with the record of row j-1, which completes
+//           row j-1 (its update is written), then the x-face at i-1/2 with
+//           the left neighbour's record taken by a warp shuffle (the flux
+//           goes to lane i-1, which needs it as its i+1/2 face, by a second
+//           shuffle).
 //
 // Registers are the limit of an FP64 flux kernel (a flux evaluation holds
 // about 60 live doubles), so what a lane carries from one row to the next --
-// row j-1's record, partial residual, input state and volume -- waits in
-// shared memory, and the row's own-cell inputs (the next row's state, the
-// stage's auxiliary inputs) arrive there by cp.async one step ahead of use.
+// row j-1's record (its first four values are the input state), partial
+// residual and volume -- waits in shared memory, and so does the y-face flux
+// while the x-face is evaluated; the row's own-cell inputs (the next row's
+// state, the stage's auxiliary inputs) arrive there by cp.async one step
+// ahead of use. What a lane needs of its quad's descriptor in every row (the
+// signs and order of its edge contributions, the corners) is read once per
+// item into a register of flags and shared memory: read from global memory
+// row by row it was a third of the warps' waiting.
+//
+// Bound by the FP64 pipe's latency at 12 warps per SM (168 registers, no
+// spills; 128 registers and 16 warps spill 84-212 bytes a thread and are 3%
+// slower). 1024^2 cells in 16x16 patches, RK3, one session alone: 357 us per
+// step with IEEE division and square root inline, 250 us with this file's
+// arithmetic (flux_fp64.cuh) and order; with three sessions' streams
+// overlapping 309 -> 186 us per step.
 #pragma once
 
 #include "async_copy.cuh"
@@ -51,12 +61,14 @@ struct Sweep64Smem {
     static constexpr int RS = 9;                      // record: rho, rho u, rho v, rho E, u, v, p, H, sqrt(rho)
     static constexpr int edge = QPW * 4 * 2 * N * 4;  // [quad][side][first/second flux][position][field]
     static constexpr int mid = QPW * N * 4;           // [quad][column][field]: faces between rows R-1 and R
-    static constexpr int carry = (RS + 4 + 4 + 1) * 32;  // [record, partial, input state, volume][lane]
-    static constexpr int qbuf = 4 * 32;                  // next row's state [field][lane]
-    static constexpr int abuf = 8 * 32;                  // auxiliary inputs a0, a1 [field][lane]
+    static constexpr int carry = (RS + 4 + 1) * 32;   // [record, partial / y-face flux, volume][lane]
+    static constexpr int qbuf = 4 * 32;               // next row's state [field][lane]
+    static constexpr int abuf = 8 * 32;               // auxiliary inputs a0, a1 [field][lane]
+    static constexpr int corner = QPW * 8;            // the quad's corners
+    static constexpr int col0 = QPW * (N + 2) * 2;    // bilinear nodes (0, row), row = 0..N
     static constexpr int o_edge = 0, o_mid = o_edge + edge, o_carry = o_mid + mid, o_q = o_carry + carry,
-                         o_a = o_q + qbuf;
-    static constexpr int per_warp = o_a + abuf;
+                         o_a = o_q + qbuf, o_corner = o_a + abuf, o_col0 = o_corner + corner;
+    static constexpr int per_warp = o_col0 + col0;
     static constexpr size_t bytes(int warps) { return sizeof(double) * (size_t)per_warp * (size_t)warps; }
 };
 
@@ -82,8 +94,7 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
     const int i = l % N, h = l / N;
     const long long stride = a.stride;
     const double scale_factor = 2.0 / (double)N;
-    const double xi0 = scale_factor * (double)i - 1.0;        // nodes at column i
-    const double xi1 = scale_factor * (double)(i + 1) - 1.0;  // ... and i+1
+    const double xi1 = scale_factor * (double)(i + 1) - 1.0;  // nodes at column i+1
 
     double *wsm = sm64 + (size_t)w * S::per_warp;
     double(*sedge)[4][2][N][4] = reinterpret_cast<double(*)[4][2][N][4]>(wsm + S::o_edge);
@@ -91,7 +102,9 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
     double *car = wsm + S::o_carry + lane;  // slot c at car[32 c]
     double *qb = wsm + S::o_q + lane;       // field f at qb[32 f]
     double *ab = wsm + S::o_a + lane;       // a0 field f at ab[32 f], a1 at ab[32 (4 + f)]
-    enum { kPart = RS, kQ = RS + 4, kVol = RS + 8 };
+    double *g = wsm + S::o_corner + 8 * sub;
+    double *c0 = wsm + S::o_col0 + 2 * (N + 2) * sub;  // node (0, row) at c0[2 row]
+    enum { kPart = RS, kVol = RS + 4 };
 
     const double dt = sweep_step_dt(a);
     double my_dt_min = a.dt_cap;
@@ -112,7 +125,6 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
         const bool valid = QPW == 1 || item * QPW + sub < a.nquad;
         const int quad = valid ? item * QPW + sub : item * QPW;
         const QuadDesc &qd = a.quads[quad];
-        const double *g = qd.corner;
         const double *Qq = a.qin + (long long)quad * NN;
         auto load_rec = [&](const double *base, int cell, double P[RS]) {
             double q[4];
@@ -125,6 +137,26 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
         for (int f = 0; f < 4; ++f) cp_async8(qb + 32 * f, Qq + f * stride + (R * h) * N + i);
         cp_async_commit();
         cp_async_commit();  // (no auxiliary group before the first row)
+        if (l < 8) g[l] = qd.corner[l];
+        // what the rows need of the sides, as bits: this lane's corner takes
+        // its y-side's contribution before its x-side's (bit 0: bottom,
+        // bit 1: top), side s adds its flux (bit 2 + s; else subtracts it),
+        // side s is a coarse hanging edge (bit 6 + s)
+        unsigned flags = 0;
+        {
+            const int sx = i == 0 ? 0 : 1;
+            const int rx = qd.side[sx].rank;
+#pragma unroll
+            for (int s = 0; s < 4; ++s) {
+                const int kind = qd.side[s].kind;
+                if (kind == kSideBoundary || (s & 1)) flags |= 4u << s;
+                if (kind == kSideCoarseHang) flags |= 64u << s;
+                if (s >= 2 && qd.side[s].rank < rx) flags |= 1u << (s - 2);
+            }
+        }
+        __syncwarp();
+        // the nodes of column 0 (lane l computes row l; the last row lane 0)
+        if (l <= N) bilinear_node(g, -1.0, scale_factor * (double)l - 1.0, c0[2 * l], c0[2 * l + 1]);
 
         // ---------------- edges: round 0 sides 0 / 1, round 1 sides 2 / 3
 #pragma unroll 1
@@ -157,7 +189,7 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
                         Lr[c] = (s & 1) ? Po[c] : Pn[c];
                         Rr[c] = (s & 1) ? Pn[c] : Po[c];
                     }
-                    roe_flux_prim_fp64(Lr, Rr, n0, n1, fl);
+                    roe_flux_prim_fp64<2>(Lr, Rr, n0, n1, fl);
 #pragma unroll
                     for (int f = 0; f < 4; ++f) sedge[sub][s][k][m][f] = fl[f];
                 }
@@ -174,8 +206,8 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
                 const double eta = scale_factor * (double)R - 1.0;
                 double x1, y1, x2, y2;
                 bilinear_node(g, xi1, eta, x1, y1);
-                bilinear_node(g, xi0, eta, x2, y2);
-                roe_flux_prim_fp64(P, O, y2 - y1, x1 - x2, fl);
+                bilinear_node(g, scale_factor * (double)i - 1.0, eta, x2, y2);
+                roe_flux_prim_fp64<1>(P, O, y2 - y1, x1 - x2, fl);
 #pragma unroll
                 for (int f = 0; f < 4; ++f) smid[sub][i][f] = fl[f];
             }
@@ -189,7 +221,7 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
             const int sy = (j == 0) ? 2 : (j == N - 1) ? 3 : -1;
             if (sx < 0 && sy < 0) return;
             int first = sx, second = sy;
-            if (sx >= 0 && sy >= 0 && qd.side[sy].rank < qd.side[sx].rank) {
+            if (sx >= 0 && sy >= 0 && (flags >> (sy - 2) & 1u)) {
                 first = sy;
                 second = sx;
             }
@@ -197,12 +229,11 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
             for (int pass = 0; pass < 2; ++pass) {
                 const int s = pass == 0 ? first : second;
                 if (s < 0) continue;
-                const int kind = qd.side[s].kind;
                 const int m = (s < 2) ? j : i;
-                const bool hang = kind == kSideCoarseHang;
+                const bool hang = flags >> (6 + s) & 1u;
                 const double *F = sedge[sub][s][0][m];
                 const double *F2 = sedge[sub][s][1][m];
-                if (kind == kSideBoundary || (s & 1)) {
+                if (flags >> (2 + s) & 1u) {
 #pragma unroll
                     for (int f = 0; f < 4; ++f) {
                         r[f] = r[f] + F[f];
@@ -223,14 +254,14 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
         auto finish = [&](int jr, const double *gup) {
             const long long gi = (long long)quad * NN + jr * N + i;
             const double vol = car[32 * kVol];
-            double kv[4], qn[4], q0v[4];
+            double r[4], kv[4], qn[4], q0v[4];
 #pragma unroll
             for (int f = 0; f < 4; ++f) {
                 const double p = car[32 * (kPart + f)];
-                const double r = gup ? p + gup[f] : p;
-                kv[f] = (r / vol) * -1.0;
-                q0v[f] = car[32 * (kQ + f)];
+                r[f] = gup ? p + gup[f] : p;
+                q0v[f] = car[32 * f];
             }
+            residual_rate(r, vol, kv);
             if (!valid) return;
             auto A0 = [&](int f) -> double { return ab[32 * f]; };
             auto A1 = [&](int f) -> double { return ab[32 * (4 + f)]; };
@@ -265,21 +296,30 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
         // ---------------- sweep over the lane's R rows. cp.async groups in
         // flight at the start of step t: the state of row j (issued one step
         // earlier) and the auxiliary inputs of row j-1.
+        //
+        // node (i+1, row) of the lane, from the corners; node (i, row) is the
+        // left lane's, and lane 0's comes from column 0's table
+        auto nodes = [&](int row, double &x0, double &y0, double &x1, double &y1) {
+            bilinear_node(g, xi1, scale_factor * (double)row - 1.0, x1, y1);
+            x0 = __shfl_up_sync(FULL, x1, 1, N);
+            y0 = __shfl_up_sync(FULL, y1, 1, N);
+            const double ex = c0[2 * row], ey = c0[2 * row + 1];
+            x0 = i == 0 ? ex : x0;
+            y0 = i == 0 ? ey : y0;
+        };
         double xa, ya, xb, yb;  // nodes (i, j) and (i+1, j) of the current row
-        {
-            const double eta = scale_factor * (double)(R * h) - 1.0;
-            bilinear_node(g, xi0, eta, xa, ya);
-            bilinear_node(g, xi1, eta, xb, yb);
-        }
+        nodes(R * h, xa, ya, xb, yb);
 #pragma unroll 1
         for (int t = 0; t < R; ++t) {
             const int j = R * h + t;
             cp_async_wait_group<1>();  // row j's state has landed
-            double q4[4];
-#pragma unroll
-            for (int f = 0; f < 4; ++f) q4[f] = qb[32 * f];
             double P[RS];
-            cell_prims_fp64(q4, P);
+            {
+                double q4[4];
+#pragma unroll
+                for (int f = 0; f < 4; ++f) q4[f] = qb[32 * f];
+                cell_prims_fp64(q4, P);
+            }
             // the next row's state into the buffer just read (the record
             // above consumed it)
             if (t < R - 1) {
@@ -287,79 +327,63 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
                 for (int f = 0; f < 4; ++f) cp_async8(qb + 32 * f, Qq + f * stride + (j + 1) * N + i);
             }
             cp_async_commit();
-            // nodes (i, j+1), (i+1, j+1), the cell's volume and x-face normal
-            double xc, yc, xd, yd;
-            {
-                const double eta = scale_factor * (double)(j + 1) - 1.0;
-                bilinear_node(g, xi0, eta, xc, yc);
-                bilinear_node(g, xi1, eta, xd, yd);
-            }
-            const double vol = subcell_volume(xa, ya, xb, yb, xc, yc, xd, yd);
-            double r[4];
-            // k = 0: x-face at i-1/2, nodes (i, j) -> (i, j+1), the left
-            //        neighbour's record (lane i = 0's is an edge face);
-            // k = 1: y-face at j-1/2, nodes (i+1, j) -> (i, j), row j-1's
-            //        record, which completes row j-1
-            const int nk = (t > 0) ? 2 : 1;
-#pragma unroll 1
-            for (int k = 0; k < nk; ++k) {
-                double A[RS];
-                double n0, n1;
-                if (k == 0) {
+            // y-face at j-1/2, nodes (i+1, j) -> (i, j), row j-1's record:
+            // completes row j-1, whose partial residual makes room for it
+            if (t > 0) {
+                double A[RS], G[4];
 #pragma unroll
-                    for (int c = 0; c < RS; ++c) A[c] = __shfl_up_sync(FULL, P[c], 1, N);
-                    n0 = yc - ya;
-                    n1 = xa - xc;
-                } else {
+                for (int c = 0; c < RS; ++c) A[c] = car[32 * c];
+                roe_flux_prim_fp64<1>(A, P, ya - yb, xb - xa, G);
+                cp_async_wait_group<1>();  // row j-1's auxiliary inputs
+                finish(j - 1, G);
 #pragma unroll
-                    for (int c = 0; c < RS; ++c) A[c] = car[32 * c];
-                    n0 = ya - yb;
-                    n1 = xb - xa;
-                }
-                double F[4];
-                roe_flux_prim_fp64(A, P, n0, n1, F);
-                if (k == 0) {
-                    double Fr[4];
-#pragma unroll
-                    for (int f = 0; f < 4; ++f) Fr[f] = __shfl_down_sync(FULL, F[f], 1, N);
-#pragma unroll
-                    for (int f = 0; f < 4; ++f) r[f] = 0.0;
-                    edge_sum(j, r);
-                    // interior x-faces only (lane 0's low and lane N-1's high
-                    // face are edge faces, summed above): each sum is
-                    // formed and kept or dropped by a select, not a branch
-#pragma unroll
-                    for (int f = 0; f < 4; ++f) {
-                        const double rl = r[f] - F[f];
-                        r[f] = i > 0 ? rl : r[f];
-                        const double rr = r[f] + Fr[f];
-                        r[f] = i < N - 1 ? rr : r[f];
-                    }
-                } else {
-#pragma unroll
-                    for (int f = 0; f < 4; ++f) r[f] = r[f] - F[f];
-                    cp_async_wait_group<1>();  // row j-1's auxiliary inputs
-                    finish(j - 1, F);
-                }
-            }
-            if (t == 0 && h == 1) {
-#pragma unroll
-                for (int f = 0; f < 4; ++f) r[f] = r[f] - smid[sub][i][f];
+                for (int f = 0; f < 4; ++f) car[32 * (kPart + f)] = G[f];
             }
             fetch_aux(j);
-            // carry row j to the next step
+            // carry row j's record to the next step
 #pragma unroll
             for (int c = 0; c < RS; ++c) car[32 * c] = P[c];
+            // nodes (i, j+1), (i+1, j+1), the cell's volume and the x-face at
+            // i-1/2, nodes (i, j) -> (i, j+1), the left neighbour's record
+            // (lane i = 0's is an edge face)
+            double n0, n1;
+            {
+                double xc, yc, xd, yd;
+                nodes(j + 1, xc, yc, xd, yd);
+                car[32 * kVol] = subcell_volume(xa, ya, xb, yb, xc, yc, xd, yd);
+                n0 = yc - ya;
+                n1 = xa - xc;
+                xa = xc;
+                ya = yc;
+                xb = xd;
+                yb = yd;
+            }
+            double F[4];
+            {
+                double A[RS];
+#pragma unroll
+                for (int c = 0; c < RS; ++c) A[c] = __shfl_up_sync(FULL, P[c], 1, N);
+                roe_flux_prim_fp64<0>(A, P, n0, n1, F);
+            }
+            double Fr[4], r[4];
+#pragma unroll
+            for (int f = 0; f < 4; ++f) Fr[f] = __shfl_down_sync(FULL, F[f], 1, N);
+#pragma unroll
+            for (int f = 0; f < 4; ++f) r[f] = 0.0;
+            edge_sum(j, r);
+            // interior faces only (lane 0's low and lane N-1's high x-face
+            // and the quad's low y-face are edge faces, summed above): each
+            // sum is formed and kept or dropped by a select, not a branch
 #pragma unroll
             for (int f = 0; f < 4; ++f) {
-                car[32 * (kPart + f)] = r[f];
-                car[32 * (kQ + f)] = q4[f];
+                const double rl = r[f] - F[f];
+                r[f] = i > 0 ? rl : r[f];
+                const double rr = r[f] + Fr[f];
+                r[f] = i < N - 1 ? rr : r[f];
+                const double G = t > 0 ? car[32 * (kPart + f)] : smid[sub][i][f];
+                const double rg = r[f] - G;
+                car[32 * (kPart + f)] = t > 0 || h == 1 ? rg : r[f];
             }
-            car[32 * kVol] = vol;
-            xa = xc;
-            ya = yc;
-            xb = xd;
-            yb = yd;
         }
         // the half's top row: the face between rows R-1 and R (h = 0) or the
         // patch's top edge, already summed (h = 1)
