@@ -483,17 +483,19 @@ bool quads_are_rectangles(const amrgpu_session *s)
 // pair, each running a serial sweep) gives way to the first block kernel
 // when the mesh has too few quads to occupy the GPU with sweep warps
 // (fewer than 1024 warps: measured slower on 256-1024 quads, faster from
-// 2048 warps on).
+// 2048 warps on); the smallest meshes take the entry marked for them.
 const StageLaunch *default_launch(int form, int n, int nquad)
 {
     const StageLaunch *tab;
     const int cnt = (form == AMRGPU_FORM_FP32_FLUX) ? stage_table_fp32(&tab) : stage_table_fp64(&tab);
-    const StageLaunch *first = nullptr, *block = nullptr;
+    const StageLaunch *first = nullptr, *block = nullptr, *small = nullptr;
     for (int i = 0; i < cnt; ++i) {
         if (tab[i].n != n) continue;
         if (!first) first = &tab[i];
         if (!block && !tab[i].sweep) block = &tab[i];
+        if (!small && nquad <= tab[i].small_quads) small = &tab[i];
     }
+    if (small) return small;
     if (first && first->sweep && block) {
         const int qpw = first->qpb / (first->threads / 32);
         const long long warps = (nquad + qpw - 1) / qpw;

@@ -121,6 +121,11 @@ const void *cfl_kernel_fp64(int n)
     StageLaunch{N, QPB, T, MINB, StageSmem<N, QPB, false>::total,                              \
                 (const void *)stage_kernel<N, QPB, T, MINB, false, FluxOpsFP64>}
 
+// ... the default up to Q quads
+#define AMRGPU_STAGE64_SMALL(N, QPB, T, MINB, Q)                                                         \
+    StageLaunch{N, QPB, T, MINB, StageSmem<N, QPB, false>::total,                                        \
+                (const void *)stage_kernel<N, QPB, T, MINB, false, FluxOpsFP64>, 0, {nullptr, nullptr, nullptr}, -1, Q}
+
 // row-sweep kernels: one warp per 16x16 quad or per two 8x8 quads
 #define AMRGPU_SWEEP64_16(W, MINB)                                                                      \
     StageLaunch{16, W, 32 * (W), MINB, Sweep64Smem<16>::bytes(W), (const void *)sweep64_16_kernel<W, MINB>, 1,  \
@@ -136,12 +141,20 @@ const void *cfl_kernel_fp64(int n)
 // Per patch size the first entry is the default launch (a row sweep gives
 // way to the size's first block kernel on meshes too small to fill the GPU
 // with sweep warps); the autotuner picks among all entries of the size.
+//
+// A mesh that leaves SMs idle is bound by one block's own latency, so its
+// quads go one to a block with a thread per face (8x8: 144 faces). Per RK3
+// stage in a graph: 64 quads of 8x8 9.9 -> 6.3 us, 256 quads 11.0 -> 6.9 us,
+// 512 quads 11.7 -> 10.9 us (two rounds; the tuner's choice there is 96
+// threads at four blocks per SM, 8.3 us), 1024 quads 11.9 -> 18.3 us; 64
+// quads of 16x16 9.1 -> 8.0 us, 192 quads 10.3 -> 13.2 us. Hence the limits:
+// as many quads as blocks are resident, two per SM and one per SM.
 static const StageLaunch kTable64[] = {
     AMRGPU_SWEEP64_16(4, 3),  // 168 registers, 12 warps per SM
     AMRGPU_SWEEP64_16(4, 4),  // 128 registers, 16 warps per SM
     AMRGPU_SWEEP64_16(2, 8),
     AMRGPU_STAGE64(16, 1, 288, 2),
-    AMRGPU_STAGE64(16, 1, 288, 1),
+    AMRGPU_STAGE64_SMALL(16, 1, 288, 1, 148),
     AMRGPU_STAGE64(16, 2, 576, 1),
     AMRGPU_STAGE64(16, 1, 256, 2),
     AMRGPU_SWEEP64_8(4, 3),   // two 8x8 quads per warp
@@ -149,6 +162,8 @@ static const StageLaunch kTable64[] = {
     AMRGPU_STAGE64(8, 4, 288, 2),
     AMRGPU_STAGE64(8, 2, 160, 3),
     AMRGPU_STAGE64(8, 4, 576, 1),
+    AMRGPU_STAGE64_SMALL(8, 1, 160, 2, 296),
+    AMRGPU_STAGE64(8, 1, 96, 4),
     AMRGPU_STAGE64(4, 8, 160, 3),
     AMRGPU_STAGE64(4, 16, 320, 2),
     AMRGPU_STAGE64(2, 16, 96, 4),
