@@ -8,25 +8,30 @@
 // hpc_amr_tag_feature, amr_external.h:92), which also labels its training
 // data and judges it at run time.
 //
-// Data flow of one training step (batch B, rows = patches):
-//   gather   X[B x 400], X^T[400 x B], y[B]        from the device dataset
-//   fwd1     Z1 = X W1^T + b1,  H1 = gelu(Z1)      (also H1^T)
-//   fwd2     Z2 = H1 W2^T + b2, H2 = gelu(Z2)      (also H2^T)
-//   fwd3     L  = H2 W3^T + b3                     (3 logits, padded to 16)
-//   loss     dL = softmax(L) - onehot(y)           (also dL^T), CE partials
-//   bwd3     dZ2 = (dL W3) * gelu'(Z2)             (also dZ2^T)
-//   bwd2     dZ1 = (dZ2 W2) * gelu'(Z1)^T          (transposed only)
-//   wgrad    dW1 = dZ1^T X, dW2^T = H1^T dZ2, dW3^T = H2^T dL   (split over B)
-//   bias     db = column sums of dZ1, dZ2, dL
-//   adamw    FP32 master update, BF16 copies W and W^T refreshed
-// Every GEMM is C[M x N] = A[M x K] B[N x K]^T with both operands K-major,
-// which is why the forward and backward epilogues also write transposes.
+// A training step (batch B, rows = patches) is three launches:
+//   mlp_tile_kernel   per 128 rows, everything that needs only those rows:
+//       Z1 = X W1^T + b1,  H1 = gelu(Z1);  Z2 = H1 W2^T + b2, H2 = gelu(Z2)
+//       L  = H2 W3^T + b3 (3 logits, padded to 16), dL = softmax(L) - onehot
+//       dZ2 = (dL W3) * gelu'(Z2),  dZ1 = (dZ2 W2) * gelu'(Z1)
+//   mlp_wgrad_kernel  dW1 = dZ1^T X, dW2^T = H1^T dZ2, dW3^T = H2^T dL as
+//       partial sums over 256 rows, db = column sums of dZ1, dZ2, dL
+//   mlp_adamw_kernel  FP32 master update, BF16 copies W and W^T refreshed
+// Inference is the first half of mlp_tile_kernel and an argmax.
+//
+// The sizes are small (7 GFLOP a batch of 8192), so a step is bound by
+// launches, by latency and by passes over memory between them, not by the
+// tensor cores. One kernel per GEMM, with operands staged chunk by chunk and
+// transposed copies for the second operand's layout, took 21 launches and
+// 283 us a batch; a tile that stays in shared and tensor memory, and
+// operands read K-major or MN-major from the same row-major copy, take
+// @@TRAIN@@.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "amrgpu_internal.h"
@@ -39,198 +44,486 @@ namespace amrgpu {
 
 using bf16 = __nv_bfloat16;
 
-enum Epi : int { kEpiHidden = 0, kEpiLogits = 1, kEpiBackHidden = 2, kEpiPartial = 3 };
+// gelu(x) = 0.5 x t and gelu'(x) = 0.5 t + x phi(x), with t = 1 + erf(x / sqrt 2)
+__device__ __forceinline__ float gelu_t(float x) { return 1.0f + erff(x * 0.70710678118654752f); }
+__device__ __forceinline__ float gelu_f(float x, float t) { return 0.5f * x * t; }
+__device__ __forceinline__ float gelu_grad_f(float x, float t)
+{
+    return 0.5f * t + x * 0.39894228040143268f * expf(-0.5f * x * x);
+}
 
-struct GemmArgs {
-    const bf16 *A;      // M x K, row stride lda (elements)
-    long long lda;
-    const bf16 *B;      // N x K, row stride ldb
-    long long ldb;
-    int M, N, K;        // N a multiple of 16, K of 8 (rows are read in 16-byte pieces)
-    int k_per_split;    // K range of one blockIdx.z (multiple of 16)
-    const float *bias;  // [N]                                (hidden, logits)
-    float *zout;        // hidden: Z [M x N] or null; logits: [M x N]; partial: [splits][M x N]
-    const float *zin;   // back-hidden: Z [M x N] for gelu'
-    bf16 *hout;         // [M x N] row-major, or null
-    bf16 *houtT;        // [N x ldt], or null
-    long long ldt;
-    int *err;           // error flags (bounded wait gave up)
+// 16 floats -> 16 BF16 as two 16-byte pieces
+__device__ __forceinline__ void pack_bf16(const float v[16], uint4 out[2])
+{
+    alignas(16) bf16 h[16];
+#pragma unroll
+    for (int k = 0; k < 16; ++k) h[k] = __float2bfloat16_rn(v[k]);
+    out[0] = reinterpret_cast<const uint4 *>(h)[0];
+    out[1] = reinterpret_cast<const uint4 *>(h)[1];
+}
+
+// Arguments of mlp_tile_kernel. Row b of the batch is row perm[b] (perm null:
+// b) of X and y. Training writes H1, H2, dZ1, dZ2, dL (row-major, B rows) and
+// per 32 rows the loss sum and the correct predictions; logits [B x 16] and
+// classes [B] are written where given.
+struct TileArgs {
+    const bf16 *X;
+    const int *perm;
+    const int *y;
+    int B;
+    const bf16 *W1, *W2, *W3, *W2T, *W3T;
+    const float *b1, *b2, *b3;
+    float *logits;
+    int *cls;
+    bf16 *H1, *H2, *dZ1, *dZ2, *dL;
+    double *loss;
+    int *correct;
+    int *err;  // error flags (a bounded wait gave up)
 };
 
-__device__ __forceinline__ float gelu_f(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
+// Shared memory of mlp_tile_kernel, in bytes. X and W1 fill it until the
+// first GEMM is done; what comes after lives in their place.
+struct TileSmem {
+    static constexpr int x = 0, xw1 = 128 * kFeatIn * 2;
+    static constexpr int w1 = x + xw1;
+    static constexpr int w2 = w1 + xw1, w3 = w2 + kH2 * kH1 * 2;
+    static constexpr int bar = w3 + kOutPad * kH2 * 2;
+    static constexpr int rows = bar + 16;  // row index of each of the 128 rows
+    static constexpr int total = rows + 128 * 4;
+    // in X's place
+    static constexpr int h1 = x, t1 = h1 + 128 * kH1 * 2;  // t1: [column][row]
+    static_assert(t1 + 128 * kH1 * 4 <= w1, "H1 and its GELU terms fit where X was");
+    // in W1's place
+    static constexpr int h2 = w1, t2 = h2 + 128 * kH2 * 2;
+    static constexpr int dl = t2 + 128 * kH2 * 4, dz2 = dl + 128 * kOutPad * 2;
+    static constexpr int w2t = dz2 + 128 * kH2 * 2, w3t = w2t + kH1 * kH2 * 2;
+    static_assert(w3t + kH2 * kOutPad * 2 <= w2, "the backward operands fit where W1 was");
+};
 
-__device__ __forceinline__ float gelu_grad_f(float x)
+constexpr int kTileThreads = 512;
+
+// Rows [0, rows) of a K-major operand of `chunks` 16-byte pieces a row,
+// row stride ld elements, into core matrices at dst by cp.async; eight rows
+// of a piece are neighbours, so a warp moves 64 contiguous bytes of eight rows.
+template <int T>
+__device__ __forceinline__ void stage_kmajor(unsigned char *dst, const bf16 *src, int rows, int chunks, int ld)
 {
-    return 0.5f * (1.0f + erff(x * 0.70710678118654752f)) + x * 0.39894228040143268f * expf(-0.5f * x * x);
+    for (int t = threadIdx.x; t < rows * chunks; t += T) {
+        const int r7 = t & 7, c = (t >> 3) % chunks, r8 = (t >> 3) / chunks;
+        cp_async16(dst + (r8 * chunks + c) * 128 + r7 * 16, src + (long long)(8 * r8 + r7) * ld + 8 * c);
+    }
 }
 
-constexpr int kGemmKC = 64;  // K elements staged per chunk
-
-template <int NT>
-constexpr size_t gemm_smem_bytes()
+// D (+)= A B^T over `steps` K = 16 steps, K-major operands of core-matrix
+// rows of `chunks` pieces, from piece c0 on
+__device__ __forceinline__ void issue_kmajor(uint32_t d, const unsigned char *a, const unsigned char *b, int chunks,
+                                             int c0, int steps, uint32_t idesc, bool first)
 {
-    return size_t(128 + NT) * kGemmKC * 2 + 64;
+    for (int k = 0; k < steps; ++k) {
+        const uint32_t off = (uint32_t)(c0 + 2 * k) * 128u;
+        umma_bf16_ss(d, umma_desc(smem_u32(a) + off, 128, (uint32_t)chunks * 128u),
+                     umma_desc(smem_u32(b) + off, 128, (uint32_t)chunks * 128u), idesc, (first && k == 0) ? 0u : 1u);
+    }
 }
 
-// One CTA = 128 rows of C (one TMEM lane each) x NT columns, over the K
-// range of its blockIdx.z. 4 warps: all stage operands, thread 0 issues the
-// MMAs, every warp drains its 32 TMEM lanes in the epilogue.
-template <int NT, int EPI>
-__global__ void __launch_bounds__(128) mlp_gemm_kernel(const GemmArgs a)
+// One CTA = 128 rows of the batch. 16 warps: warp w reads TMEM lanes (rows)
+// 32 (w % 4) .. and a quarter w / 4 of the columns; thread 0 issues the MMAs.
+template <bool TRAIN>
+__global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArgs a)
 {
-    static_assert(NT % 16 == 0 && NT >= 16 && NT <= 256, "UMMA N for M = 128");
-    constexpr int KC = kGemmKC;
-    constexpr uint32_t NCOLS = NT <= 32 ? 32 : NT <= 64 ? 64 : NT <= 128 ? 128 : 256;
-    extern __shared__ __align__(128) unsigned char mlp_smem[];
-    unsigned char *sA = mlp_smem;
-    unsigned char *sB = mlp_smem + 128 * KC * 2;
-    uint64_t *bar = reinterpret_cast<uint64_t *>(mlp_smem + (128 + NT) * KC * 2);
+    using S = TileSmem;
+    constexpr uint32_t kCols = TRAIN ? 512 : 256;
+    // accumulators: Z1, Z2 and the logits stay for the backward pass
+    constexpr uint32_t dZ1c = 0, dZ2c = 128, dLc = 192, dB2c = 256, dB1c = 320;
+    constexpr int kGroups = 5, kGroupChunks = kFeatIn / 8 / kGroups;
+    extern __shared__ __align__(128) unsigned char sm[];
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::bar);
     uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 1);
-
+    int *srow = reinterpret_cast<int *>(sm + S::rows);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * 128, n0 = blockIdx.y * NT;
-    const int kbeg = blockIdx.z * a.k_per_split;
-    const int kend = min(a.K, kbeg + a.k_per_split);
+    const int m0 = blockIdx.x * 128;
 
-    if (warp == 0) tmem_alloc(tslot, NCOLS);
+    if (warp == 0) tmem_alloc(tslot, kCols);
     if (tid == 0) {
         mbar_init(bar, 1);
         fence_mbar_init();
     }
+    stage_launch_gate();
+    if (tid < 128) srow[tid] = m0 + tid < a.B ? (a.perm ? a.perm[m0 + tid] : m0 + tid) : -1;
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *tslot;
-    const uint32_t idesc = umma_idesc_bf16_f32(128, NT);
+
+    // ---------------- operands: X and W1 in K groups of 80, then W2 and W3
+    for (int g = 0; g < kGroups; ++g) {
+        const int c0 = g * kGroupChunks;
+        for (int t = tid; t < 2 * 128 * kGroupChunks; t += kTileThreads) {
+            const bool isx = t < 128 * kGroupChunks;
+            const int u = isx ? t : t - 128 * kGroupChunks;
+            const int r7 = u & 7, c = c0 + (u >> 3) % kGroupChunks, r8 = (u >> 3) / kGroupChunks;
+            const int r = 8 * r8 + r7;
+            unsigned char *dst = sm + (isx ? S::x : S::w1) + (r8 * (kFeatIn / 8) + c) * 128 + r7 * 16;
+            const int row = isx ? srow[r] : r;
+            if (row >= 0) cp_async16(dst, (isx ? a.X : a.W1) + (long long)row * kFeatIn + 8 * c);
+            else *reinterpret_cast<uint4 *>(dst) = make_uint4(0u, 0u, 0u, 0u);
+        }
+        cp_async_commit();
+    }
+    stage_kmajor<kTileThreads>(sm + S::w2, a.W2, kH2, kH1 / 8, kH1);
+    stage_kmajor<kTileThreads>(sm + S::w3, a.W3, kOutPad, kH2 / 8, kH2);
+    cp_async_commit();
 
     unsigned phase = 0;
     int ok = 1;
-    for (int k0 = kbeg; k0 < kend && ok; k0 += KC) {
-        const int kc = min(KC, kend - k0);
-        for (int t = tid; t < 128 * (KC / 8); t += 128) {
-            const int r = t / (KC / 8), c8 = t % (KC / 8);
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (m0 + r < a.M && c8 * 8 < kc)
-                v = *reinterpret_cast<const uint4 *>(a.A + (long long)(m0 + r) * a.lda + k0 + c8 * 8);
-            *reinterpret_cast<uint4 *>(sA + ((r >> 3) * (KC / 8) + c8) * 128 + (r & 7) * 16) = v;
-        }
-        for (int t = tid; t < NT * (KC / 8); t += 128) {
-            const int r = t / (KC / 8), c8 = t % (KC / 8);
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (n0 + r < a.N && c8 * 8 < kc)
-                v = *reinterpret_cast<const uint4 *>(a.B + (long long)(n0 + r) * a.ldb + k0 + c8 * 8);
-            *reinterpret_cast<uint4 *>(sB + ((r >> 3) * (KC / 8) + c8) * 128 + (r & 7) * 16) = v;
-        }
-        fence_async_smem();
-        __syncthreads();
-        if (tid == 0) {
-            tc_fence_after();
-            const uint32_t abase = smem_u32(sA), bbase = smem_u32(sB);
-            // a K range ending inside a 16-element step is zero-filled above
-            for (int kk = 0; kk < (kc + 15) / 16; ++kk) {
-                const uint64_t ad = umma_desc_kmajor(abase + kk * 256, 128, KC * 16);
-                const uint64_t bd = umma_desc_kmajor(bbase + kk * 256, 128, KC * 16);
-                umma_bf16_ss(tmem, ad, bd, idesc, (k0 > kbeg || kk > 0) ? 1u : 0u);
-            }
-            umma_commit(bar);
-        }
-        // the next chunk overwrites the operands only after these MMAs finish
+    // the MMAs issued so far have finished (bounded wait); false ends the block
+    auto done = [&]() -> bool {
         if (!mbar_wait_bounded(bar, phase, kWaitLimit)) ok = 0;
         phase ^= 1u;
         ok = __syncthreads_and(ok);
-    }
-    if (!ok) {
-        // gave up waiting: report, let anything in flight finish (bounded),
-        // release the tensor memory and leave without writing results
+        tc_fence_after();
+        return ok != 0;
+    };
+    // generic writes (and landed copies) of every thread, then the MMAs
+    auto publish = [&]() {
+        fence_async_smem();
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+    };
+    auto give_up = [&]() {
+        // report, and release the tensor memory without writing results;
+        // the MMAs in flight get another bounded wait
         if (tid == 0) atomicOr(a.err, kFlagTimeout);
+        cp_async_wait_all();
         mbar_wait_bounded(bar, phase ^ 1u, kWaitLimit);
         tc_fence_before();
         __syncthreads();
-        if (warp == 0) tmem_dealloc(tmem, NCOLS);
+        if (warp == 0) tmem_dealloc(tmem, kCols);
+    };
+
+    // ---------------- Z1 = X W1^T
+    auto group = [&](int g) {
+        publish();
+        if (tid == 0)
+            issue_kmajor(tmem + dZ1c, sm + S::x, sm + S::w1, kFeatIn / 8, g * kGroupChunks, kGroupChunks / 2,
+                         umma_idesc_bf16_f32(128, kH1), g == 0);
+    };
+    cp_async_wait_group<5>();
+    group(0);
+    cp_async_wait_group<4>();
+    group(1);
+    cp_async_wait_group<3>();
+    group(2);
+    cp_async_wait_group<2>();
+    group(3);
+    cp_async_wait_group<1>();
+    group(4);
+    if (tid == 0) umma_commit(bar);
+    if (!done()) return give_up();
+    // the backward operands into W1's place, while H1 is made
+    if (TRAIN) {
+        stage_kmajor<kTileThreads>(sm + S::w2t, a.W2T, kH1, kH2 / 8, kH2);
+        stage_kmajor<kTileThreads>(sm + S::w3t, a.W3T, kH2, kOutPad / 8, kOutPad);
+    }
+    cp_async_commit();
+
+    const int r = 32 * (warp & 3) + lane, cg = warp >> 2;
+    const int row = m0 + r;
+    const bool rv = row < a.B;
+    const uint32_t tl = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
+    float *t1 = reinterpret_cast<float *>(sm + S::t1), *t2 = reinterpret_cast<float *>(sm + S::t2);
+    // 16 columns from nb on of a hidden layer: + bias, GELU, the next GEMM's
+    // operand (and its copy for the weight gradients)
+    auto hidden = [&](uint32_t dcol, const float *bias, int nb, int width, unsigned char *tile, float *tt, bf16 *out) {
+        float v[16];
+        tmem_ld16(tl + dcol + (uint32_t)nb, v);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            v[k] += bias[nb + k];
+            const float t = gelu_t(v[k]);
+            if (TRAIN) tt[(nb + k) * 128 + r] = t;
+            v[k] = gelu_f(v[k], t);
+        }
+        uint4 h[2];
+        pack_bf16(v, h);
+        unsigned char *dst = tile + ((r >> 3) * (width / 8) + nb / 8) * 128 + (r & 7) * 16;
+        *reinterpret_cast<uint4 *>(dst) = h[0];
+        *reinterpret_cast<uint4 *>(dst + 128) = h[1];
+        if (TRAIN && rv) {
+            uint4 *o = reinterpret_cast<uint4 *>(out + (long long)row * width + nb);
+            o[0] = h[0];
+            o[1] = h[1];
+        }
+    };
+#pragma unroll 1
+    for (int nb = 32 * cg; nb < 32 * cg + 32; nb += 16) hidden(dZ1c, a.b1, nb, kH1, sm + S::h1, t1, a.H1);
+
+    // ---------------- Z2 = H1 W2^T
+    cp_async_wait_group<1>();  // W2 and W3 (the backward operands may be under way)
+    publish();
+    if (tid == 0) {
+        issue_kmajor(tmem + dZ2c, sm + S::h1, sm + S::w2, kH1 / 8, 0, kH1 / 16, umma_idesc_bf16_f32(128, kH2), true);
+        umma_commit(bar);
+    }
+    if (!done()) return give_up();
+    hidden(dZ2c, a.b2, 16 * cg, kH2, sm + S::h2, t2, a.H2);
+
+    // ---------------- L = H2 W3^T
+    publish();
+    if (tid == 0) {
+        issue_kmajor(tmem + dLc, sm + S::h2, sm + S::w3, kH2 / 8, 0, kH2 / 16, umma_idesc_bf16_f32(128, kOutPad), true);
+        umma_commit(bar);
+    }
+    if (!done()) return give_up();
+    if (cg == 0) {
+        float v[16];
+        tmem_ld16(tl + dLc, v);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) v[k] += a.b3[k];
+        if (a.logits && rv) {
+            float4 *dst = reinterpret_cast<float4 *>(a.logits + (long long)row * kOutPad);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+        }
+        const float l0 = v[0], l1 = v[1], l2 = v[2];
+        const int arg = (l0 >= l1 && l0 >= l2) ? 0 : (l1 >= l2 ? 1 : 2);
+        if (a.cls && rv) a.cls[row] = arg;
+        if (TRAIN) {
+            // softmax cross-entropy on the 3 logits: dL = softmax - onehot
+            // (not divided by B; the optimiser scales), zero in the padding
+            double loss = 0.0;
+            int corr = 0;
+            float g[16] = {};
+            if (rv) {
+                const float mx = fmaxf(l0, fmaxf(l1, l2));
+                const float e0 = expf(l0 - mx), e1 = expf(l1 - mx), e2 = expf(l2 - mx);
+                const float s = e0 + e1 + e2;
+                const int yy = a.y[srow[r]];
+                const float ly = yy == 0 ? l0 : yy == 1 ? l1 : l2;
+                loss = (double)(mx + logf(s) - ly);
+                corr = arg == yy;
+                g[0] = e0 / s - (yy == 0 ? 1.0f : 0.0f);
+                g[1] = e1 / s - (yy == 1 ? 1.0f : 0.0f);
+                g[2] = e2 / s - (yy == 2 ? 1.0f : 0.0f);
+            }
+            uint4 h[2];
+            pack_bf16(g, h);
+            unsigned char *dst = sm + S::dl + (r >> 3) * 256 + (r & 7) * 16;
+            *reinterpret_cast<uint4 *>(dst) = h[0];
+            *reinterpret_cast<uint4 *>(dst + 128) = h[1];
+            if (rv) {
+                uint4 *o = reinterpret_cast<uint4 *>(a.dL + (long long)row * kOutPad);
+                o[0] = h[0];
+                o[1] = h[1];
+            }
+            loss = warp_sum(loss);
+            corr = __reduce_add_sync(0xffffffffu, corr);
+            if (lane == 0) {
+                a.loss[blockIdx.x * 4 + warp] = loss;
+                a.correct[blockIdx.x * 4 + warp] = corr;
+            }
+        }
+    }
+    if (TRAIN) {
+        // ---------------- dZ2 = (dL W3) * gelu'(Z2)
+        cp_async_wait_all();
+        publish();
+        if (tid == 0) {
+            issue_kmajor(tmem + dB2c, sm + S::dl, sm + S::w3t, kOutPad / 8, 0, 1, umma_idesc_bf16_f32(128, kH2), true);
+            umma_commit(bar);
+        }
+        if (!done()) return give_up();
+        // 16 columns from nb on of a hidden layer's gradient
+        auto back = [&](uint32_t dcol, uint32_t zcol, const float *bias, int nb, int width, unsigned char *tile,
+                        const float *tt, bf16 *out) {
+            float v[16], z[16];
+            tmem_ld16(tl + dcol + (uint32_t)nb, v);
+            tmem_ld16(tl + zcol + (uint32_t)nb, z);
+#pragma unroll
+            for (int k = 0; k < 16; ++k) v[k] *= gelu_grad_f(z[k] + bias[nb + k], tt[(nb + k) * 128 + r]);
+            uint4 h[2];
+            pack_bf16(v, h);
+            if (tile) {
+                unsigned char *dst = tile + ((r >> 3) * (width / 8) + nb / 8) * 128 + (r & 7) * 16;
+                *reinterpret_cast<uint4 *>(dst) = h[0];
+                *reinterpret_cast<uint4 *>(dst + 128) = h[1];
+            }
+            if (rv) {
+                uint4 *o = reinterpret_cast<uint4 *>(out + (long long)row * width + nb);
+                o[0] = h[0];
+                o[1] = h[1];
+            }
+        };
+        back(dB2c, dZ2c, a.b2, 16 * cg, kH2, sm + S::dz2, t2, a.dZ2);
+        // ---------------- dZ1 = (dZ2 W2) * gelu'(Z1)
+        publish();
+        if (tid == 0) {
+            issue_kmajor(tmem + dB1c, sm + S::dz2, sm + S::w2t, kH2 / 8, 0, kH2 / 16, umma_idesc_bf16_f32(128, kH1),
+                         true);
+            umma_commit(bar);
+        }
+        if (!done()) return give_up();
+#pragma unroll 1
+        for (int nb = 32 * cg; nb < 32 * cg + 32; nb += 16) back(dB1c, dZ1c, a.b1, nb, kH1, nullptr, t1, a.dZ1);
+    }
+    tc_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_dealloc(tmem, kCols);
+}
+
+// Arguments of mlp_wgrad_kernel: the tile kernel's outputs, X as there.
+struct WgradArgs {
+    const bf16 *X;
+    const int *perm;
+    int B;
+    const bf16 *H1, *H2, *dZ1, *dZ2, *dL;
+    float *P1, *P2, *P3;  // per 256 rows: dW1 [128 x 400], dW2^T [128 x 64], dW3^T [64 x 16]
+    float *gb;            // bias gradients, summed over the batch
+    int *err;
+};
+
+constexpr int kWgradThreads = 256;
+constexpr int kWgradRoles = 7;            // five fifths of dW1, dW2, dW3
+constexpr int kWgradN1 = kFeatIn / 5;     // columns of a dW1 role
+constexpr int kBiasBlocks = (kH1 + kH2 + kOutPad) / 8;
+constexpr int kBiasRows = 4096;           // rows staged at a time
+constexpr int kWgradA = kWgradK * 128 * 2, kWgradB = kWgradK * kWgradN1 * 2;
+constexpr int kWgradSmem = kWgradA + kWgradB + 16;
+static_assert(kBiasRows * 16 + 32 * 8 * 4 <= kWgradA + kWgradB, "bias rows fit the operands' space");
+
+// The weight gradients' partial sums: one CTA per 256 rows and role, C[M x N]
+// = A^T B with A [256 x M] and B [256 x N] row-major, i.e. both operands
+// MN-major: a core matrix is 8 rows of 16 bytes along M (or N), the leading
+// offset goes to the next 8 rows, the stride offset to the next 16 bytes. The
+// last kBiasBlocks CTAs sum 8 columns each of dZ1, dZ2, dL over the whole
+// batch, each row in lane b % 32's sum, then the lanes as a shuffle tree does.
+__global__ void __launch_bounds__(kWgradThreads, 2) mlp_wgrad_kernel(const WgradArgs a)
+{
+    extern __shared__ __align__(128) unsigned char sm[];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int splits = (a.B + kWgradK - 1) / kWgradK;
+    stage_launch_gate();
+    if ((int)blockIdx.x >= splits * kWgradRoles) {
+        const int u0 = 8 * ((int)blockIdx.x - splits * kWgradRoles);
+        const bf16 *src;
+        int ld;
+        if (u0 < kH1) { src = a.dZ1 + u0; ld = kH1; }
+        else if (u0 < kH1 + kH2) { src = a.dZ2 + (u0 - kH1); ld = kH2; }
+        else { src = a.dL + (u0 - kH1 - kH2); ld = kOutPad; }
+        const int u = tid & 7, l = tid >> 3;
+        float s = 0.0f;
+        for (int b0 = 0; b0 < a.B; b0 += kBiasRows) {
+            const int nb = min(kBiasRows, a.B - b0);
+            for (int k = tid; k < nb; k += kWgradThreads) cp_async16(sm + k * 16, src + (long long)(b0 + k) * ld);
+            cp_async_commit();
+            cp_async_wait_all();
+            __syncthreads();
+            const bf16 *rows = reinterpret_cast<const bf16 *>(sm);
+#pragma unroll 8
+            for (int k = l; k < nb; k += 32) s += __bfloat162float(rows[k * 8 + u]);
+            __syncthreads();
+        }
+        float *p = reinterpret_cast<float *>(sm + kBiasRows * 16);
+        p[l * 8 + u] = s;
+        for (int o = 16; o > 0; o >>= 1) {
+            __syncthreads();
+            if (l < o) p[l * 8 + u] += p[(l + o) * 8 + u];
+        }
+        if (l == 0) a.gb[u0 + u] = p[u];
         return;
     }
+
+    constexpr uint32_t kCols = 128;
+    uint64_t *bar = reinterpret_cast<uint64_t *>(sm + kWgradA + kWgradB);
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 1);
+    const int z = blockIdx.x / kWgradRoles, role = blockIdx.x % kWgradRoles;
+    const int k0 = z * kWgradK, kc = min(kWgradK, a.B - k0), kr = (kc + 15) / 16 * 16;
+    // M, N in 16-byte pieces, the operands' rows and where the result goes
+    const int ma = role < 6 ? 16 : 8, nb = role < 5 ? kWgradN1 / 8 : role == 5 ? kH2 / 8 : kOutPad / 8;
+    const bf16 *A = role < 5 ? a.dZ1 : role == 5 ? a.H1 : a.H2;
+    const bf16 *Bm = role < 5 ? a.X + role * kWgradN1 : role == 5 ? a.dZ2 : a.dL;
+    const int ldb = role < 5 ? kFeatIn : role == 5 ? kH2 : kOutPad;
+    if (warp == 0) tmem_alloc(tslot, kCols);
+    if (tid == 0) {
+        mbar_init(bar, 1);
+        fence_mbar_init();
+    }
+    unsigned char *sA = sm, *sB = sm + kWgradA;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    // rows in four groups, each its own copy group
+    for (int g = 0; g < 4; ++g) {
+        const int ke = min(kr, 64 * (g + 1));
+        for (int t = tid; t < 64 * 16; t += kWgradThreads) {
+            const int k = 64 * g + (t & 7) + 8 * (t >> 7), c = (t >> 3) & 15;
+            if (k >= ke) continue;
+            unsigned char *dst = sA + ((k >> 3) * 16 + c) * 128 + (k & 7) * 16;
+            if (k < kc && c < ma) cp_async16(dst, A + (long long)(k0 + k) * (8 * ma) + 8 * c);
+            else *reinterpret_cast<uint4 *>(dst) = zero;
+        }
+        for (int t = tid; t < 64 * nb; t += kWgradThreads) {
+            const int k = 64 * g + (t & 7) + 8 * ((t >> 3) / nb), c = (t >> 3) % nb;
+            if (k >= ke) continue;
+            unsigned char *dst = sB + ((k >> 3) * nb + c) * 128 + (k & 7) * 16;
+            if (k < kc) {
+                const int row = role < 5 && a.perm ? a.perm[k0 + k] : k0 + k;
+                cp_async16(dst, Bm + (long long)row * ldb + 8 * c);
+            } else {
+                *reinterpret_cast<uint4 *>(dst) = zero;
+            }
+        }
+        cp_async_commit();
+    }
+    const uint32_t idesc = umma_idesc_bf16_f32(128, 8 * nb) | kUmmaMnMajorA | kUmmaMnMajorB;
+    uint32_t tmem = 0;
+    auto group = [&](int g) {
+        fence_async_smem();
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+        tmem = *tslot;
+        if (tid == 0) {
+            for (int k = 64 * g; k < min(kr, 64 * (g + 1)); k += 16)
+                umma_bf16_ss(tmem, umma_desc(smem_u32(sA) + (uint32_t)(k >> 3) * 2048u, 2048, 128),
+                             umma_desc(smem_u32(sB) + (uint32_t)((k >> 3) * nb) * 128u, (uint32_t)nb * 128u, 128),
+                             idesc, k > 0 ? 1u : 0u);
+        }
+    };
+    cp_async_wait_group<3>();
+    group(0);
+    cp_async_wait_group<2>();
+    group(1);
+    cp_async_wait_group<1>();
+    group(2);
+    cp_async_wait_group<0>();
+    group(3);
+    if (tid == 0) umma_commit(bar);
+    int ok = mbar_wait_bounded(bar, 0, kWaitLimit) ? 1 : 0;
+    ok = __syncthreads_and(ok);
     tc_fence_after();
-    const bool any = kend > kbeg;
-    const int row = m0 + warp * 32 + lane;
-    const bool rv = row < a.M;
-#pragma unroll 1
-    for (int c0 = 0; c0 < NT; c0 += 16) {
-        float v[16];
-        tmem_ld16(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, v);
-        if (!any) {
-#pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] = 0.0f;
-        }
-        const int nb = n0 + c0;
-        if (nb >= a.N) continue;
-        if (EPI == kEpiHidden || EPI == kEpiLogits) {
-#pragma unroll
-            for (int k = 0; k < 16; ++k) v[k] += a.bias[nb + k];
-            if (rv && a.zout) {
-                float4 *dst = reinterpret_cast<float4 *>(a.zout + (long long)row * a.N + nb);
+    if (!ok) {
+        if (tid == 0) atomicOr(a.err, kFlagTimeout);
+        mbar_wait_bounded(bar, 0, kWaitLimit);
+    } else {
+        const int row = 32 * (warp & 3) + lane;
+        float *out;
+        int ldo;
+        if (role < 5) { out = a.P1 + ((long long)z * kH1 + row) * kFeatIn + role * kWgradN1; ldo = kH1; }
+        else if (role == 5) { out = a.P2 + ((long long)z * kH1 + row) * kH2; ldo = kH1; }
+        else { out = a.P3 + ((long long)z * kH2 + row) * kOutPad; ldo = kH2; }
+        for (int c = 16 * (warp >> 2); c < 8 * nb; c += 32) {
+            float v[16];
+            tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)c, v);
+            if (row < ldo) {
+                float4 *dst = reinterpret_cast<float4 *>(out + c);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-            }
-            if (EPI == kEpiHidden) {
-#pragma unroll
-                for (int k = 0; k < 16; ++k) v[k] = gelu_f(v[k]);
-            }
-        } else if (EPI == kEpiBackHidden) {
-            if (rv) {
-                const float4 *zp = reinterpret_cast<const float4 *>(a.zin + (long long)row * a.N + nb);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const float4 z = zp[k];
-                    v[4 * k] *= gelu_grad_f(z.x);
-                    v[4 * k + 1] *= gelu_grad_f(z.y);
-                    v[4 * k + 2] *= gelu_grad_f(z.z);
-                    v[4 * k + 3] *= gelu_grad_f(z.w);
-                }
-            }
-        } else {  // kEpiPartial
-            if (rv) {
-                float4 *dst = reinterpret_cast<float4 *>(a.zout + ((long long)blockIdx.z * a.M + row) * a.N + nb);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) dst[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
-            }
-            continue;
-        }
-        if (EPI == kEpiHidden || EPI == kEpiBackHidden) {
-            if (rv && a.hout) {
-                alignas(16) bf16 h[16];
-#pragma unroll
-                for (int k = 0; k < 16; ++k) h[k] = __float2bfloat16_rn(v[k]);
-                uint4 *dst = reinterpret_cast<uint4 *>(a.hout + (long long)row * a.N + nb);
-                dst[0] = reinterpret_cast<const uint4 *>(h)[0];
-                dst[1] = reinterpret_cast<const uint4 *>(h)[1];
-            }
-            if (rv && a.houtT) {
-#pragma unroll
-                for (int k = 0; k < 16; ++k) a.houtT[(long long)(nb + k) * a.ldt + row] = __float2bfloat16_rn(v[k]);
             }
         }
     }
     tc_fence_before();
     __syncthreads();
-    if (warp == 0) tmem_dealloc(tmem, NCOLS);
-}
-
-template <int NT, int EPI>
-static cudaError_t launch_gemm(const GemmArgs &a, int splits, cudaStream_t st)
-{
-    const void *k = (const void *)mlp_gemm_kernel<NT, EPI>;
-    // cap residency at what tensor memory holds (512 columns per SM), so an
-    // allocation never waits on a CTA that is not yet resident
-    constexpr uint32_t ncols = NT <= 32 ? 32 : NT <= 64 ? 64 : NT <= 128 ? 128 : 256;
-    constexpr int per_sm = 512 / ncols;
-    size_t smem = gemm_smem_bytes<NT>();
-    const size_t cap = (size_t)220 * 1024 / per_sm + 1024;
-    if (smem < cap) smem = cap;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    dim3 grid((a.M + 127) / 128, (a.N + NT - 1) / NT, splits);
-    void *args[] = {const_cast<GemmArgs *>(&a)};
-    return cudaLaunchKernel(k, grid, dim3(128), args, smem, st);
+    if (warp == 0) tmem_dealloc(tmem, kCols);
 }
 
 // ---------------------------------------------------------------- features
@@ -369,156 +662,6 @@ __global__ void jump_kernel(const double *rho, const QuadDesc *quads, const int 
     if (lane == 0) jump[w] = J;
 }
 
-// ---------------------------------------------------------------- training kernels
-
-// rows perm[b0 .. b0+B) of the dataset -> X[B x 400], X^T[400 x B], y[B]
-__global__ void gather_kernel(const bf16 *Xall, const int *yall, const int *perm, int b0, int B, bf16 *X, bf16 *XT,
-                              int *y)
-{
-    const int b = blockIdx.x;
-    const int src = perm[b0 + b];
-    for (int k = threadIdx.x; k < kFeatIn; k += blockDim.x) {
-        const bf16 v = Xall[(long long)src * kFeatIn + k];
-        X[(long long)b * kFeatIn + k] = v;
-        XT[(long long)k * B + b] = v;
-    }
-    if (threadIdx.x == 0) y[b] = yall[src];
-}
-
-// Softmax cross-entropy on the first 3 of 16 logit columns:
-// dL = softmax - onehot (not divided by B; the optimiser scales), written
-// row-major and transposed (padding columns zero); per-block partial sums of
-// the loss and of correct predictions.
-__global__ void __launch_bounds__(256) softmax_ce_kernel(const float *L, const int *y, int B, bf16 *dL, bf16 *dLT,
-                                                         double *loss_part, int *correct_part)
-{
-    __shared__ double sl[8];
-    __shared__ int sc[8];
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    double loss = 0.0;
-    int corr = 0;
-    if (b < B) {
-        const float l0 = L[(long long)b * kOutPad], l1 = L[(long long)b * kOutPad + 1], l2 = L[(long long)b * kOutPad + 2];
-        const float mx = fmaxf(l0, fmaxf(l1, l2));
-        const float e0 = expf(l0 - mx), e1 = expf(l1 - mx), e2 = expf(l2 - mx);
-        const float s = e0 + e1 + e2;
-        const float p[3] = {e0 / s, e1 / s, e2 / s};
-        const int yy = y[b];
-        const float ly = yy == 0 ? l0 : yy == 1 ? l1 : l2;
-        loss = (double)(mx + logf(s) - ly);
-        const int arg = (l0 >= l1 && l0 >= l2) ? 0 : (l1 >= l2 ? 1 : 2);
-        corr = arg == yy;
-        for (int c = 0; c < kOutPad; ++c) {
-            const float g = c < 3 ? p[c] - (c == yy ? 1.0f : 0.0f) : 0.0f;
-            dL[(long long)b * kOutPad + c] = __float2bfloat16_rn(g);
-            dLT[(long long)c * B + b] = __float2bfloat16_rn(g);
-        }
-    }
-    loss = warp_sum(loss);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) corr += __shfl_xor_sync(0xffffffffu, corr, o);
-    if ((threadIdx.x & 31) == 0) {
-        sl[threadIdx.x >> 5] = loss;
-        sc[threadIdx.x >> 5] = corr;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double tl = 0.0;
-        int tc = 0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
-            tl += sl[w];
-            tc += sc[w];
-        }
-        loss_part[blockIdx.x] = tl;
-        correct_part[blockIdx.x] = tc;
-    }
-}
-
-// Row sums of a transposed gradient G^T[rows x B] (bias gradients), one
-// warp per row, fixed order.
-__global__ void rowsum_kernel(const bf16 *GT, int rows, int B, float *out)
-{
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-    if (w >= rows) return;
-    float s = 0.0f;
-    for (int b = lane; b < B; b += 32) s += __bfloat162float(GT[(long long)w * B + b]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (lane == 0) out[w] = s;
-}
-
-// Gradient of one parameter tensor element (o, i) of a [rows x cols]
-// weight: sum over splits of the weight-gradient GEMM partials, read
-// transposed when the GEMM produced W^T, or a finished sum (biases); times
-// 1/B (the loss kernel leaves dL unscaled).
-struct GradSrc {
-    const float *part;  // [splits][prow x pcol] GEMM partials, or null
-    const float *gsum;  // finished sums, or null
-    int splits, prow, pcol;
-    int transposed;
-    int rows, cols;
-};
-
-__device__ __forceinline__ float grad_of(const GradSrc &g, int idx, float inv_b)
-{
-    const int o = idx / g.cols, i = idx % g.cols;
-    float s = 0.0f;
-    if (g.part) {
-        const long long off = g.transposed ? (long long)i * g.pcol + o : (long long)o * g.pcol + i;
-        for (int k = 0; k < g.splits; ++k) s += g.part[(long long)k * g.prow * g.pcol + off];
-    } else {
-        s = g.gsum[idx];
-    }
-    return s * inv_b;
-}
-
-// AdamW (decoupled weight decay) on FP32 master weights; refreshes the BF16
-// copy W (row-major [rows x cols]) and W^T ([cols x ldt]) used by the GEMMs.
-struct AdamArgs {
-    GradSrc g;
-    float *w, *m, *v;
-    __nv_bfloat16 *wb, *wbT;
-    float *fcopy;  // FP32 copy (padded bias of the logits), or null
-    int ldt;
-    float inv_b, lr, wd, b1, b2, eps, c1, c2;  // c1 = 1/(1-b1^t), c2 = 1/(1-b2^t)
-};
-
-__global__ void adamw_kernel(const AdamArgs a)
-{
-    const int n = a.g.rows * a.g.cols;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
-        const float g = grad_of(a.g, idx, a.inv_b);
-        const float m = a.b1 * a.m[idx] + (1.0f - a.b1) * g;
-        const float v = a.b2 * a.v[idx] + (1.0f - a.b2) * g * g;
-        a.m[idx] = m;
-        a.v[idx] = v;
-        float w = a.w[idx];
-        w -= a.lr * ((m * a.c1) / (sqrtf(v * a.c2) + a.eps) + a.wd * w);
-        a.w[idx] = w;
-        const int o = idx / a.g.cols, i = idx % a.g.cols;
-        const __nv_bfloat16 wb = __float2bfloat16_rn(w);
-        if (a.wb) a.wb[idx] = wb;
-        if (a.wbT) a.wbT[(long long)i * a.ldt + o] = wb;
-        if (a.fcopy) a.fcopy[idx] = w;
-    }
-}
-
-__global__ void grad_kernel(const GradSrc g, float inv_b, float *out)
-{
-    const int n = g.rows * g.cols;
-    for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x)
-        out[idx] = grad_of(g, idx, inv_b);
-}
-
-// argmax of the 3 logits -> indicator tag (class index)
-__global__ void argmax_kernel(const float *L, int B, int *cls)
-{
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    const float l0 = L[(long long)b * kOutPad], l1 = L[(long long)b * kOutPad + 1], l2 = L[(long long)b * kOutPad + 2];
-    cls[b] = (l0 >= l1 && l0 >= l2) ? 0 : (l1 >= l2 ? 1 : 2);
-}
-
 // plain three-class label from the jump: refine (1) when J >= tol, coarsen
 // (0) when J < lo_frac * tol, keep (2) in between. cover: merged into the
 // label already there, keeping the finer demand (refine if either asks for
@@ -537,9 +680,99 @@ __global__ void label_kernel(const double *J, int n, double tol, double lo_frac,
     cls[k] = c;
 }
 
-// ---------------------------------------------------------------- host side
 
-static int grid1(long long n, int block) { return (int)std::max<long long>(1, std::min<long long>((n + block - 1) / block, 148LL * 32)); }
+// ---------------------------------------------------------------- optimiser
+
+// The parameter tensors in flat order (W1, b1, W2, b2, W3, b3) and where
+// each one's gradient is after the weight-gradient kernel.
+struct GradArgs {
+    const float *P1, *P2, *P3, *gb;
+    int splits;
+    float inv_b;  // the loss kernel leaves dL unscaled
+};
+
+constexpr int kOffB1 = kH1 * kFeatIn, kOffW2 = kOffB1 + kH1, kOffB2 = kOffW2 + kH2 * kH1, kOffW3 = kOffB2 + kH2,
+              kOffB3 = kOffW3 + kOut * kH2;
+
+// Gradient of flat parameter idx: a weight's is the sum over the partials in
+// order, read transposed where they hold W^T.
+__device__ __forceinline__ float grad_of(const GradArgs &g, int idx)
+{
+    const float *p;
+    int step;
+    if (idx < kOffB1) {
+        p = g.P1 + idx;
+        step = kH1 * kFeatIn;
+    } else if (idx < kOffW2) {
+        return g.gb[idx - kOffB1] * g.inv_b;
+    } else if (idx < kOffB2) {
+        const int k = idx - kOffW2, o = k / kH1, i = k % kH1;
+        p = g.P2 + i * kH2 + o;
+        step = kH1 * kH2;
+    } else if (idx < kOffW3) {
+        return g.gb[kH1 + idx - kOffB2] * g.inv_b;
+    } else if (idx < kOffB3) {
+        const int k = idx - kOffW3, o = k / kH2, i = k % kH2;
+        p = g.P3 + i * kOutPad + o;
+        step = kH2 * kOutPad;
+    } else {
+        return g.gb[kH1 + kH2 + idx - kOffB3] * g.inv_b;
+    }
+    float s = 0.0f;
+#pragma unroll 8
+    for (int k = 0; k < g.splits; ++k) s += p[(long long)k * step];
+    return s * g.inv_b;
+}
+
+// AdamW (decoupled weight decay, on weights only) on the FP32 master
+// parameters; refreshes the BF16 copies W (row-major) and W^T and the padded
+// FP32 b3 that the tile kernel reads.
+struct AdamArgs {
+    GradArgs g;
+    float *w, *m, *v;
+    bf16 *W1, *W2, *W3, *W2T, *W3T;
+    float *b3p;
+    float lr, wd, b1, b2, eps, c1, c2;  // c1 = 1/(1-b1^t), c2 = 1/(1-b2^t)
+};
+
+__global__ void __launch_bounds__(256) mlp_adamw_kernel(const AdamArgs a)
+{
+    stage_launch_gate();
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= kMlpParams) return;
+    const bool weight = idx < kOffB1 || (idx >= kOffW2 && idx < kOffB2) || (idx >= kOffW3 && idx < kOffB3);
+    const float g = grad_of(a.g, idx);
+    const float m = a.b1 * a.m[idx] + (1.0f - a.b1) * g;
+    const float v = a.b2 * a.v[idx] + (1.0f - a.b2) * g * g;
+    a.m[idx] = m;
+    a.v[idx] = v;
+    float w = a.w[idx];
+    const float wd = weight ? a.wd : 0.0f;
+    w -= a.lr * ((m * a.c1) / (sqrtf(v * a.c2) + a.eps) + wd * w);
+    a.w[idx] = w;
+    const bf16 wb = __float2bfloat16_rn(w);
+    if (idx < kOffB1) {
+        a.W1[idx] = wb;
+    } else if (idx >= kOffW2 && idx < kOffB2) {
+        const int k = idx - kOffW2, o = k / kH1, i = k % kH1;
+        a.W2[k] = wb;
+        a.W2T[i * kH2 + o] = wb;
+    } else if (idx >= kOffW3 && idx < kOffB3) {
+        const int k = idx - kOffW3, o = k / kH2, i = k % kH2;
+        a.W3[k] = wb;
+        a.W3T[i * kOutPad + o] = wb;
+    } else if (idx >= kOffB3) {
+        a.b3p[idx - kOffB3] = w;
+    }
+}
+
+__global__ void __launch_bounds__(256) mlp_grad_kernel(const GradArgs g, float *out)
+{
+    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx < kMlpParams) out[idx] = grad_of(g, idx);
+}
+
+// ---------------------------------------------------------------- host side
 
 cudaError_t mlp_launch_features(int n, const double *q, long long stride, const QuadDesc *quads, int nquad, bf16 *X,
                                 cudaStream_t st)
@@ -588,13 +821,26 @@ bool dalloc(T **p, size_t n, std::vector<void *> &own)
 
 // Offsets of the flat FP32 parameter vector: W1 [128x400], b1, W2 [64x128],
 // b2, W3 [3x64], b3.
-const int kParamOff[7] = {0,
-                          kH1 * kFeatIn,
-                          kH1 * kFeatIn + kH1,
-                          kH1 * kFeatIn + kH1 + kH2 * kH1,
-                          kH1 * kFeatIn + kH1 + kH2 * kH1 + kH2,
-                          kH1 * kFeatIn + kH1 + kH2 * kH1 + kH2 + kOut * kH2,
-                          kMlpParams};
+const int kParamOff[7] = {0, kOffB1, kOffW2, kOffB2, kOffW3, kOffB3, kMlpParams};
+
+// A launch that may be scheduled while its predecessor in the stream drains
+// (the kernel waits on the device, stage_launch_gate).
+template <class Args>
+cudaError_t launch_after(const void *kernel, int grid, int threads, size_t smem, const Args &a, cudaStream_t st)
+{
+    cudaLaunchConfig_t lc = {};
+    lc.gridDim = dim3((unsigned)grid);
+    lc.blockDim = dim3((unsigned)threads);
+    lc.dynamicSmemBytes = smem;
+    lc.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    lc.attrs = at;
+    lc.numAttrs = 1;
+    void *args[] = {const_cast<Args *>(&a)};
+    return cudaLaunchKernelExC(&lc, kernel, args);
+}
 
 }  // namespace
 
@@ -612,13 +858,16 @@ void MlpState::release()
     cudaFree(jump);
     cudaFree(which);
     cudaFree(jcls);
+    cudaFree(stats);
+    cap_stats = 0;
+    stats = nullptr;
     Xall = nullptr;
     yall = nullptr;
     perm = nullptr;
     jump = nullptr;
     which = nullptr;
     jcls = nullptr;
-    cap_batch = 0;
+    cap_batch = cap_train = 0;
     cap_data = n_data = cap_perm = 0;
     cap_judge = 0;
 }
@@ -691,31 +940,46 @@ bool MlpState::refresh_bf16()
            cudaMemset(err, 0, sizeof(int)) == cudaSuccess;
 }
 
-bool MlpState::ensure_batch(int B)
+// Buffers for batches of B rows: features, labels, logits and classes, and
+// with `train` what the weight gradients are made from.
+bool MlpState::ensure_batch(int B, bool train)
 {
-    if (B <= cap_batch) return true;
+    if (B <= cap_batch && (!train || B <= cap_train)) return true;
     // twice the old capacity at least (rows stay a multiple of 128): a mesh
     // that grows a few quads per regrid reallocates rarely
-    B = std::max(B, 2 * cap_batch);
+    if (B > cap_batch) B = std::max(B, 2 * cap_batch);
+    else B = cap_batch;
+    train = train || cap_train > 0;
     cudaStreamSynchronize(stream);
     for (void *p : batch_owned) cudaFree(p);
     batch_owned.clear();
-    cap_batch = 0;
+    cap_batch = cap_train = 0;
     auto &o = batch_owned;
     const size_t b = size_t(B);
     const size_t splits = (b + kWgradK - 1) / kWgradK;
-    const size_t blocks = (b + 255) / 256;
-    const bool ok =
-        dalloc(&X, b * kFeatIn, o) && dalloc(&XT, b * kFeatIn, o) && dalloc(&y, b, o) && dalloc(&Z1, b * kH1, o) &&
-        dalloc(&H1, b * kH1, o) && dalloc(&H1T, b * kH1, o) && dalloc(&Z2, b * kH2, o) && dalloc(&H2, b * kH2, o) &&
-        dalloc(&H2T, b * kH2, o) && dalloc(&Lg, b * kOutPad, o) && dalloc(&dL, b * kOutPad, o) &&
-        dalloc(&dLT, b * kOutPad, o) && dalloc(&dZ2, b * kH2, o) && dalloc(&dZ2T, b * kH2, o) &&
-        dalloc(&dZ1T, b * kH1, o) && dalloc(&P1, splits * kH1 * kFeatIn, o) && dalloc(&P2, splits * kH1 * kH2, o) &&
-        dalloc(&P3, splits * kH2 * kOutPad, o) && dalloc(&gb, size_t(kH1 + kH2 + kOutPad), o) &&
-        dalloc(&gflat, size_t(kMlpParams), o) && dalloc(&loss_part, blocks, o) && dalloc(&corr_part, blocks, o) &&
-        dalloc(&cls, b, o);
+    bool ok = dalloc(&X, b * kFeatIn, o) && dalloc(&y, b, o) && dalloc(&Lg, b * kOutPad, o) && dalloc(&cls, b, o);
+    if (ok && train)
+        ok = dalloc(&H1, b * kH1, o) && dalloc(&H2, b * kH2, o) && dalloc(&dZ1, b * kH1, o) &&
+             dalloc(&dZ2, b * kH2, o) && dalloc(&dL, b * kOutPad, o) && dalloc(&P1, splits * kH1 * kFeatIn, o) &&
+             dalloc(&P2, splits * kH1 * kH2, o) && dalloc(&P3, splits * kH2 * kOutPad, o) &&
+             dalloc(&gb, size_t(kH1 + kH2 + kOutPad), o) && dalloc(&gflat, size_t(kMlpParams), o);
     if (ok) cap_batch = B;
+    if (ok && train) cap_train = B;
     return ok;
+}
+
+bool MlpState::ensure_stats(long long groups)
+{
+    if (groups <= cap_stats) return true;
+    cudaStreamSynchronize(stream);
+    cudaFree(stats);
+    stats = nullptr;
+    cap_stats = 0;
+    groups = std::max<long long>(groups, 1024);
+    if (cudaMalloc((void **)&stats, (sizeof(double) + sizeof(int)) * size_t(groups) + sizeof(double)) != cudaSuccess)
+        return false;
+    cap_stats = groups;
+    return true;
 }
 
 bool MlpState::ensure_data(long long n)
@@ -761,137 +1025,109 @@ bool MlpState::ensure_judge(int n)
     return true;
 }
 
-// Forward pass of B rows of X (device, row-major): logits into Lg; with
-// `train` also Z1, Z2, H1^T, H2^T for the backward pass.
-cudaError_t MlpState::forward(int B, bool train, cudaStream_t st)
-{
-    GemmArgs g{};
-    g.err = err;
-    // fwd1: [B x 400] x W1[128 x 400]^T
-    g.A = X; g.lda = kFeatIn; g.B = W1; g.ldb = kFeatIn; g.M = B; g.N = kH1; g.K = kFeatIn; g.k_per_split = kFeatIn;
-    g.bias = w + kParamOff[1]; g.zout = train ? Z1 : nullptr; g.hout = H1; g.houtT = train ? H1T : nullptr; g.ldt = B;
-    cudaError_t e = launch_gemm<128, kEpiHidden>(g, 1, st);
-    if (e != cudaSuccess) return e;
-    // fwd2: [B x 128] x W2[64 x 128]^T
-    g.A = H1; g.lda = kH1; g.B = W2; g.ldb = kH1; g.N = kH2; g.K = kH1; g.k_per_split = kH1;
-    g.bias = w + kParamOff[3]; g.zout = train ? Z2 : nullptr; g.hout = H2; g.houtT = train ? H2T : nullptr;
-    if ((e = launch_gemm<64, kEpiHidden>(g, 1, st)) != cudaSuccess) return e;
-    // fwd3: [B x 64] x W3[16 x 64]^T (rows 3..15 zero)
-    g.A = H2; g.lda = kH2; g.B = W3; g.ldb = kH2; g.N = kOutPad; g.K = kH2; g.k_per_split = kH2;
-    g.bias = b3p; g.zout = Lg; g.hout = nullptr; g.houtT = nullptr;
-    return launch_gemm<16, kEpiLogits>(g, 1, st);
-}
-
-cudaError_t MlpState::loss(int B, cudaStream_t st)
-{
-    softmax_ce_kernel<<<(B + 255) / 256, 256, 0, st>>>(Lg, y, B, dL, dLT, loss_part, corr_part);
-    return cudaGetLastError();
-}
-
-// Backward pass after forward(B, true) and loss(B): the weight-gradient
-// partials P1..P3 and the bias sums gb.
-cudaError_t MlpState::backward(int B, cudaStream_t st)
-{
-    GemmArgs g{};
-    g.err = err;
-    // bwd3: dH2 = dL[B x 16] W3p[16 x 64]; operand W3^T[64 x 16]
-    g.A = dL; g.lda = kOutPad; g.B = W3T; g.ldb = kOutPad; g.M = B; g.N = kH2; g.K = kOutPad; g.k_per_split = kOutPad;
-    g.zin = Z2; g.hout = dZ2; g.houtT = dZ2T; g.ldt = B;
-    cudaError_t e = launch_gemm<64, kEpiBackHidden>(g, 1, st);
-    if (e != cudaSuccess) return e;
-    // bwd2: dH1 = dZ2[B x 64] W2[64 x 128]; operand W2^T[128 x 64]
-    g.A = dZ2; g.lda = kH2; g.B = W2T; g.ldb = kH2; g.N = kH1; g.K = kH2; g.k_per_split = kH2;
-    g.zin = Z1; g.hout = nullptr; g.houtT = dZ1T;
-    if ((e = launch_gemm<128, kEpiBackHidden>(g, 1, st)) != cudaSuccess) return e;
-    // weight gradients, K = batch in slices of kWgradK rows
-    const int splits = (B + kWgradK - 1) / kWgradK;
-    GemmArgs p{};
-    p.err = err;
-    p.k_per_split = kWgradK;
-    p.K = B;
-    // dW1[128 x 400] = dZ1^T[128 x B] (X^T[400 x B])^T
-    p.A = dZ1T; p.lda = B; p.B = XT; p.ldb = B; p.M = kH1; p.N = kFeatIn; p.zout = P1;
-    if ((e = launch_gemm<80, kEpiPartial>(p, splits, st)) != cudaSuccess) return e;
-    // dW2^T[128 x 64] = H1^T[128 x B] (dZ2^T[64 x B])^T
-    p.A = H1T; p.B = dZ2T; p.M = kH1; p.N = kH2; p.zout = P2;
-    if ((e = launch_gemm<64, kEpiPartial>(p, splits, st)) != cudaSuccess) return e;
-    // dW3^T[64 x 16] = H2^T[64 x B] (dL^T[16 x B])^T
-    p.A = H2T; p.B = dLT; p.M = kH2; p.N = kOutPad; p.zout = P3;
-    if ((e = launch_gemm<16, kEpiPartial>(p, splits, st)) != cudaSuccess) return e;
-    // bias gradients: row sums of dZ1^T, dZ2^T, dL^T
-    rowsum_kernel<<<(kH1 * 32 + 255) / 256, 256, 0, st>>>(dZ1T, kH1, B, gb);
-    rowsum_kernel<<<(kH2 * 32 + 255) / 256, 256, 0, st>>>(dZ2T, kH2, B, gb + kH1);
-    rowsum_kernel<<<(kOutPad * 32 + 255) / 256, 256, 0, st>>>(dLT, kOutPad, B, gb + kH1 + kH2);
-    return cudaGetLastError();
-}
-
 namespace {
 
-// where each parameter tensor's gradient lives after backward()
-GradSrc grad_src(const MlpState &s, int t, int B)
+TileArgs tile_args(const MlpState &s, const RowSource &r, int B)
 {
-    const int splits = (B + kWgradK - 1) / kWgradK;
-    GradSrc g{};
-    g.splits = splits;
-    switch (t) {
-    case 0: g.part = s.P1; g.prow = kH1; g.pcol = kFeatIn; g.rows = kH1; g.cols = kFeatIn; break;
-    case 1: g.gsum = s.gb; g.rows = 1; g.cols = kH1; break;
-    case 2: g.part = s.P2; g.prow = kH1; g.pcol = kH2; g.transposed = 1; g.rows = kH2; g.cols = kH1; break;
-    case 3: g.gsum = s.gb + kH1; g.rows = 1; g.cols = kH2; break;
-    case 4: g.part = s.P3; g.prow = kH2; g.pcol = kOutPad; g.transposed = 1; g.rows = kOut; g.cols = kH2; break;
-    default: g.gsum = s.gb + kH1 + kH2; g.rows = 1; g.cols = kOut; break;
-    }
+    TileArgs a{};
+    a.X = r.X;
+    a.perm = r.perm;
+    a.y = r.y;
+    a.B = B;
+    a.W1 = s.W1; a.W2 = s.W2; a.W3 = s.W3; a.W2T = s.W2T; a.W3T = s.W3T;
+    a.b1 = s.w + kOffB1; a.b2 = s.w + kOffB2; a.b3 = s.b3p;
+    a.err = s.err;
+    return a;
+}
+
+GradArgs grad_args(const MlpState &s, int B)
+{
+    GradArgs g{};
+    g.P1 = s.P1; g.P2 = s.P2; g.P3 = s.P3; g.gb = s.gb;
+    g.splits = (B + kWgradK - 1) / kWgradK;
+    g.inv_b = 1.0f / (float)B;
     return g;
 }
 
+// The kernels' shared-memory opt-in, once per device.
+cudaError_t opt_in()
+{
+    static std::mutex mu;
+    static std::vector<int> done;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lk(mu);
+    if (std::find(done.begin(), done.end(), dev) != done.end()) return cudaSuccess;
+    const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
+    if ((e = cudaFuncSetAttribute((const void *)mlp_tile_kernel<false>, attr, TileSmem::total)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute((const void *)mlp_tile_kernel<true>, attr, TileSmem::total)) != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute((const void *)mlp_wgrad_kernel, attr, kWgradSmem)) != cudaSuccess) return e;
+    done.push_back(dev);
+    return cudaSuccess;
+}
+
 }  // namespace
+
+// Forward pass of B rows: logits [B x 16] and classes where given.
+cudaError_t MlpState::infer(const RowSource &r, int B, float *logits, int *classes, cudaStream_t st)
+{
+    cudaError_t e = opt_in();
+    if (e != cudaSuccess) return e;
+    TileArgs a = tile_args(*this, r, B);
+    a.logits = logits;
+    a.cls = classes;
+    return launch_after((const void *)mlp_tile_kernel<false>, (B + 127) / 128, kTileThreads, TileSmem::total, a, st);
+}
+
+// Forward and backward pass of B rows (a multiple of 8): the weight-gradient
+// partials P1..P3, the bias sums gb, and per 32 rows the loss sum and the
+// correct predictions.
+cudaError_t MlpState::gradients(const RowSource &r, int B, float *logits, double *loss, int *correct, cudaStream_t st)
+{
+    cudaError_t e = opt_in();
+    if (e != cudaSuccess) return e;
+    TileArgs a = tile_args(*this, r, B);
+    a.logits = logits;
+    a.H1 = H1; a.H2 = H2; a.dZ1 = dZ1; a.dZ2 = dZ2; a.dL = dL;
+    a.loss = loss;
+    a.correct = correct;
+    e = launch_after((const void *)mlp_tile_kernel<true>, (B + 127) / 128, kTileThreads, TileSmem::total, a, st);
+    if (e != cudaSuccess) return e;
+    WgradArgs w{};
+    w.X = r.X;
+    w.perm = r.perm;
+    w.B = B;
+    w.H1 = H1; w.H2 = H2; w.dZ1 = dZ1; w.dZ2 = dZ2; w.dL = dL;
+    w.P1 = P1; w.P2 = P2; w.P3 = P3; w.gb = gb;
+    w.err = err;
+    const int splits = (B + kWgradK - 1) / kWgradK;
+    return launch_after((const void *)mlp_wgrad_kernel, splits * kWgradRoles + kBiasBlocks, kWgradThreads, kWgradSmem,
+                        w, st);
+}
 
 cudaError_t MlpState::update(int B, float lr, float wd, cudaStream_t st)
 {
     ++step;
     const float b1 = 0.9f, b2 = 0.999f;
     AdamArgs a{};
-    a.inv_b = 1.0f / (float)B;
+    a.g = grad_args(*this, B);
+    a.w = w; a.m = m; a.v = v;
+    a.W1 = W1; a.W2 = W2; a.W3 = W3; a.W2T = W2T; a.W3T = W3T;
+    a.b3p = b3p;
     a.lr = lr;
+    a.wd = wd;
     a.b1 = b1;
     a.b2 = b2;
     a.eps = 1e-8f;
     a.c1 = (float)(1.0 / (1.0 - std::pow((double)b1, (double)step)));
     a.c2 = (float)(1.0 / (1.0 - std::pow((double)b2, (double)step)));
-    for (int t = 0; t < 6; ++t) {
-        a.g = grad_src(*this, t, B);
-        a.w = w + kParamOff[t];
-        a.m = m + kParamOff[t];
-        a.v = v + kParamOff[t];
-        a.wd = (t % 2 == 0) ? wd : 0.0f;  // no decay on biases
-        a.wb = t == 0 ? W1 : t == 2 ? W2 : t == 4 ? W3 : nullptr;
-        a.wbT = t == 2 ? W2T : t == 4 ? W3T : nullptr;
-        a.ldt = t == 2 ? kH2 : kOutPad;
-        a.fcopy = t == 5 ? b3p : nullptr;
-        const long long n = (long long)a.g.rows * a.g.cols;
-        adamw_kernel<<<grid1(n, 256), 256, 0, st>>>(a);
-    }
-    return cudaGetLastError();
+    return launch_after((const void *)mlp_adamw_kernel, (kMlpParams + 255) / 256, 256, 0, a, st);
 }
 
 cudaError_t MlpState::flat_grad(int B, cudaStream_t st)
 {
-    for (int t = 0; t < 6; ++t) {
-        const GradSrc g = grad_src(*this, t, B);
-        grad_kernel<<<grid1((long long)g.rows * g.cols, 256), 256, 0, st>>>(g, 1.0f / (float)B, gflat + kParamOff[t]);
-    }
-    return cudaGetLastError();
-}
-
-cudaError_t MlpState::gather(const int *perm_dev, int b0, int B, cudaStream_t st)
-{
-    gather_kernel<<<B, 128, 0, st>>>(Xall, yall, perm_dev, b0, B, X, XT, y);
-    return cudaGetLastError();
-}
-
-cudaError_t MlpState::argmax(int B, int *out, cudaStream_t st)
-{
-    argmax_kernel<<<(B + 255) / 256, 256, 0, st>>>(Lg, B, out);
+    mlp_grad_kernel<<<(kMlpParams + 255) / 256, 256, 0, st>>>(grad_args(*this, B), gflat);
     return cudaGetLastError();
 }
 

@@ -53,6 +53,18 @@ double judge_u01(unsigned long long seed, int q)
     return (double)(z >> 11) * (1.0 / 9007199254740992.0);
 }
 
+// total + the losses of one batch, given per 32 rows: 256 rows are summed at
+// a time, then added
+double add_losses(double total, const double *loss, long long groups)
+{
+    for (long long k = 0; k < groups; k += 8) {
+        double t = 0.0;
+        for (long long j = k; j < std::min(k + 8, groups); ++j) t += loss[j];
+        total += t;
+    }
+    return total;
+}
+
 }  // namespace
 
 extern "C" {
@@ -226,7 +238,10 @@ int amrgpu_mlp_train_epoch(amrgpu_mlp_t *m, const int *perm, long long n, int ba
             return AMRGPU_ERR_ARG;
         }
     const long long nb = n / batch;
-    if (!ms.ensure_batch(batch)) {
+    // per 32 rows: a loss sum and the correct predictions; the wait flags of
+    // the tensor-core kernels come back behind them
+    const long long per = 4LL * ((batch + 127) / 128), groups = per * std::max<long long>(nb, 1);
+    if (!ms.ensure_batch(batch, true) || !ms.ensure_stats(groups)) {
         set_error(AMRGPU_ERR_CUDA, "train: device allocation failed");
         return AMRGPU_ERR_CUDA;
     }
@@ -240,43 +255,27 @@ int amrgpu_mlp_train_epoch(amrgpu_mlp_t *m, const int *perm, long long n, int ba
     cudaStream_t st = ms.stream;
     if (!ok_cuda(cudaMemcpyAsync(ms.perm, perm, sizeof(int) * size_t(n), cudaMemcpyHostToDevice, st), "H2D perm"))
         return AMRGPU_ERR_CUDA;
-    const int blocks = (batch + 255) / 256;
-    std::vector<double> lp(size_t(blocks) * size_t(std::max<long long>(nb, 1)));
-    std::vector<int> cp(lp.size());
-    double *d_lp = nullptr;
-    int *d_cp = nullptr;
-    if (!ok_cuda(cudaMalloc(&d_lp, sizeof(double) * lp.size()), "alloc") ||
-        !ok_cuda(cudaMalloc(&d_cp, sizeof(int) * cp.size()), "alloc")) {
-        cudaFree(d_lp);
-        return AMRGPU_ERR_CUDA;
-    }
+    double *d_loss = ms.stats;
+    int *d_corr = reinterpret_cast<int *>(ms.stats + groups);
     bool ok = true;
     for (long long b = 0; b < nb && ok; ++b) {
-        ok = ok_cuda(ms.gather(ms.perm, int(b * batch), batch, st), "gather") &&
-             ok_cuda(ms.forward(batch, true, st), "forward") && ok_cuda(ms.loss(batch, st), "loss") &&
-             ok_cuda(cudaMemcpyAsync(d_lp + b * blocks, ms.loss_part, sizeof(double) * blocks, cudaMemcpyDeviceToDevice,
-                                     st),
-                     "loss partials") &&
-             ok_cuda(cudaMemcpyAsync(d_cp + b * blocks, ms.corr_part, sizeof(int) * blocks, cudaMemcpyDeviceToDevice,
-                                     st),
-                     "accuracy partials") &&
-             ok_cuda(ms.backward(batch, st), "backward") && ok_cuda(ms.update(batch, lr, weight_decay, st), "adamw");
+        const RowSource rows{ms.Xall, ms.perm + b * batch, ms.yall};
+        ok = ok_cuda(ms.gradients(rows, batch, nullptr, d_loss + b * per, d_corr + b * per, st), "gradients") &&
+             ok_cuda(ms.update(batch, lr, weight_decay, st), "adamw");
     }
+    std::vector<double> stats(size_t(groups) + size_t(groups + 1) / 2 + 1);
+    double *lp = stats.data();
+    const int *cp = reinterpret_cast<const int *>(lp + groups);
     if (ok && nb > 0)
-        ok = ok_cuda(cudaMemcpyAsync(lp.data(), d_lp, sizeof(double) * size_t(nb * blocks), cudaMemcpyDeviceToHost, st),
-                     "D2H") &&
-             ok_cuda(cudaMemcpyAsync(cp.data(), d_cp, sizeof(int) * size_t(nb * blocks), cudaMemcpyDeviceToHost, st),
+        ok = ok_cuda(cudaMemcpyAsync(lp, d_loss, (sizeof(double) + sizeof(int)) * size_t(groups), cudaMemcpyDeviceToHost,
+                                     st),
                      "D2H");
     if (ok) ok = ok_cuda(cudaStreamSynchronize(st), "sync") && check_flags(ms);
-    cudaFree(d_lp);
-    cudaFree(d_cp);
     if (!ok) return AMRGPU_ERR_CUDA;
     double tl = 0.0;
     long long tc = 0;
-    for (long long k = 0; k < nb * blocks; ++k) {
-        tl += lp[size_t(k)];
-        tc += cp[size_t(k)];
-    }
+    for (long long b = 0; b < nb; ++b) tl = add_losses(tl, lp + b * per, per);
+    for (long long k = 0; k < nb * per; ++k) tc += cp[k];
     const double rows = (double)std::max<long long>(nb * batch, 1);
     if (mean_loss) *mean_loss = tl / rows;
     if (accuracy) *accuracy = (double)tc / rows;
@@ -294,22 +293,20 @@ int amrgpu_mlp_grad(amrgpu_mlp_t *m, const uint16_t *features, const int *labels
     for (int k = 0; k < batch; ++k)
         if (labels[k] < 0 || labels[k] > 2) return AMRGPU_ERR_ARG;
     MlpState &ms = m->st;
-    if (!ms.ensure_batch(batch)) return AMRGPU_ERR_CUDA;
+    const long long groups = 4LL * ((batch + 127) / 128);
+    if (!ms.ensure_batch(batch, true) || !ms.ensure_stats(groups)) return AMRGPU_ERR_CUDA;
     cudaStream_t st = ms.stream;
     const size_t fb = sizeof(uint16_t) * size_t(batch) * kFeatIn;
-    std::vector<uint16_t> xt(size_t(batch) * kFeatIn);
-    for (int b = 0; b < batch; ++b)
-        for (int k = 0; k < kFeatIn; ++k) xt[size_t(k) * batch + b] = features[size_t(b) * kFeatIn + k];
-    const int blocks = (batch + 255) / 256;
-    std::vector<double> lp((size_t)blocks);
+    std::vector<double> lp((size_t)groups);
     std::vector<float> lg(size_t(batch) * kOutPad);
+    const RowSource rows{ms.X, nullptr, ms.y};
     bool ok = ok_cuda(cudaMemcpyAsync(ms.X, features, fb, cudaMemcpyHostToDevice, st), "H2D") &&
-              ok_cuda(cudaMemcpyAsync(ms.XT, xt.data(), fb, cudaMemcpyHostToDevice, st), "H2D") &&
               ok_cuda(cudaMemcpyAsync(ms.y, labels, sizeof(int) * size_t(batch), cudaMemcpyHostToDevice, st), "H2D") &&
-              ok_cuda(ms.forward(batch, true, st), "forward") && ok_cuda(ms.loss(batch, st), "loss") &&
-              ok_cuda(ms.backward(batch, st), "backward") && ok_cuda(ms.flat_grad(batch, st), "grad") &&
+              ok_cuda(ms.gradients(rows, batch, ms.Lg, ms.stats, reinterpret_cast<int *>(ms.stats + groups), st),
+                      "gradients") &&
+              ok_cuda(ms.flat_grad(batch, st), "grad") &&
               ok_cuda(cudaMemcpyAsync(lg.data(), ms.Lg, sizeof(float) * lg.size(), cudaMemcpyDeviceToHost, st), "D2H") &&
-              ok_cuda(cudaMemcpyAsync(lp.data(), ms.loss_part, sizeof(double) * lp.size(), cudaMemcpyDeviceToHost, st),
+              ok_cuda(cudaMemcpyAsync(lp.data(), ms.stats, sizeof(double) * lp.size(), cudaMemcpyDeviceToHost, st),
                       "D2H");
     if (ok && grad)
         ok = ok_cuda(cudaMemcpyAsync(grad, ms.gflat, sizeof(float) * kMlpParams, cudaMemcpyDeviceToHost, st), "D2H");
@@ -318,11 +315,7 @@ int amrgpu_mlp_grad(amrgpu_mlp_t *m, const uint16_t *features, const int *labels
     if (logits)
         for (int b = 0; b < batch; ++b)
             for (int c = 0; c < kOut; ++c) logits[size_t(b) * kOut + c] = lg[size_t(b) * kOutPad + c];
-    if (mean_loss) {
-        double t = 0.0;
-        for (double x : lp) t += x;
-        *mean_loss = t / batch;
-    }
+    if (mean_loss) *mean_loss = add_losses(0.0, lp.data(), groups) / batch;
     return AMRGPU_OK;
 }
 
@@ -330,13 +323,13 @@ int amrgpu_mlp_predict(amrgpu_mlp_t *m, const uint16_t *features, int batch, flo
 {
     if (!m || !features || !logits || batch <= 0) return AMRGPU_ERR_ARG;
     MlpState &ms = m->st;
-    if (!ms.ensure_batch(batch)) return AMRGPU_ERR_CUDA;
+    if (!ms.ensure_batch(batch, false)) return AMRGPU_ERR_CUDA;
     cudaStream_t st = ms.stream;
     std::vector<float> lg(size_t(batch) * kOutPad);
     bool ok = ok_cuda(cudaMemcpyAsync(ms.X, features, sizeof(uint16_t) * size_t(batch) * kFeatIn,
                                       cudaMemcpyHostToDevice, st),
                       "H2D") &&
-              ok_cuda(ms.forward(batch, false, st), "forward") &&
+              ok_cuda(ms.infer(RowSource{ms.X, nullptr, nullptr}, batch, ms.Lg, nullptr, st), "forward") &&
               ok_cuda(cudaMemcpyAsync(lg.data(), ms.Lg, sizeof(float) * lg.size(), cudaMemcpyDeviceToHost, st), "D2H") &&
               ok_cuda(cudaStreamSynchronize(st), "sync") && check_flags(ms);
     if (!ok) return AMRGPU_ERR_CUDA;
@@ -360,7 +353,7 @@ int amrgpu_session_learned_tags(amrgpu_session_t *s, amrgpu_mlp_t *m, double jud
     cudaStream_t st = (cudaStream_t)v.stream;
     if (!ok_cuda(cudaStreamSynchronize(ms.stream), "sync")) return AMRGPU_ERR_CUDA;
     const int B = ((v.nquad + 127) / 128) * 128;
-    if (!ms.ensure_batch(B) || !ms.ensure_judge(v.nquad)) {
+    if (!ms.ensure_batch(B, false) || !ms.ensure_judge(v.nquad)) {
         set_error(AMRGPU_ERR_CUDA, "learned tags: device allocation failed");
         return AMRGPU_ERR_CUDA;
     }
@@ -372,9 +365,9 @@ int amrgpu_session_learned_tags(amrgpu_session_t *s, amrgpu_mlp_t *m, double jud
     const int nj = int(which.size());
     std::vector<int> jl((size_t)nj);
     bool ok = ok_cuda(mlp_launch_features(v.n, v.q, v.stride, v.quads, v.nquad, ms.X, st), "features kernel") &&
-              ok_cuda(ms.forward(v.nquad, false, st), "forward") && ok_cuda(ms.argmax(v.nquad, ms.cls, st), "argmax") &&
+              ok_cuda(ms.infer(RowSource{ms.X, nullptr, nullptr}, v.nquad, nullptr, ms.cls, st), "forward") &&
               ok_cuda(cudaMemcpyAsync(tags, ms.cls, sizeof(int) * size_t(v.nquad), cudaMemcpyDeviceToHost, st), "D2H");
-    int launches = 5;
+    int launches = 2;
     if (ok && nj > 0) {
         ok = ok_cuda(cudaMemcpyAsync(ms.which, which.data(), sizeof(int) * size_t(nj), cudaMemcpyHostToDevice, st),
                      "H2D judge") &&

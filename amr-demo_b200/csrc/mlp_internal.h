@@ -31,6 +31,13 @@ cudaError_t mlp_launch_jump(int n, const double *rho, const QuadDesc *quads, con
 cudaError_t mlp_launch_labels(const double *J, int n, double tol, double lo_frac, int *cls, cudaStream_t st,
                               bool cover = false);
 
+// The rows of a batch: row b is row perm[b] (perm null: b) of X and y.
+struct RowSource {
+    const __nv_bfloat16 *X;
+    const int *perm;
+    const int *y;
+};
+
 struct MlpState {
     // FP32 master parameters and AdamW moments (flat: W1, b1, W2, b2, W3, b3)
     float *w = nullptr, *m = nullptr, *v = nullptr;
@@ -42,15 +49,18 @@ struct MlpState {
     long long step = 0;
     std::vector<void *> fixed_owned;
 
-    // per-batch work buffers (capacity cap_batch rows)
-    int cap_batch = 0;
-    __nv_bfloat16 *X = nullptr, *XT = nullptr, *H1 = nullptr, *H1T = nullptr, *H2 = nullptr, *H2T = nullptr;
-    __nv_bfloat16 *dL = nullptr, *dLT = nullptr, *dZ2 = nullptr, *dZ2T = nullptr, *dZ1T = nullptr;
-    float *Z1 = nullptr, *Z2 = nullptr, *Lg = nullptr, *P1 = nullptr, *P2 = nullptr, *P3 = nullptr, *gb = nullptr;
-    float *gflat = nullptr;
-    double *loss_part = nullptr;
-    int *corr_part = nullptr, *y = nullptr, *cls = nullptr;
+    // per-batch work buffers: features, labels, logits and classes (capacity
+    // cap_batch rows), and for training (cap_train rows) the layers' outputs
+    // and gradients, row-major, and the weight-gradient partials
+    int cap_batch = 0, cap_train = 0;
+    __nv_bfloat16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *dL = nullptr, *dZ2 = nullptr, *dZ1 = nullptr;
+    float *Lg = nullptr, *P1 = nullptr, *P2 = nullptr, *P3 = nullptr, *gb = nullptr, *gflat = nullptr;
+    int *y = nullptr, *cls = nullptr;
     std::vector<void *> batch_owned;
+    // per 32 rows of every batch of an epoch: loss sums, then correct
+    // predictions (ints), in one allocation
+    double *stats = nullptr;
+    long long cap_stats = 0;
 
     // device dataset of (features, plain label) pairs
     __nv_bfloat16 *Xall = nullptr;
@@ -71,16 +81,14 @@ struct MlpState {
     bool init(uint64_t seed);
     bool set_params(const float *h);
     bool refresh_bf16();
-    bool ensure_batch(int B);
+    bool ensure_batch(int B, bool train);
+    bool ensure_stats(long long groups);
     bool ensure_data(long long n);
     bool ensure_judge(int n);
-    cudaError_t gather(const int *perm_dev, int b0, int B, cudaStream_t st);
-    cudaError_t forward(int B, bool train, cudaStream_t st);
-    cudaError_t loss(int B, cudaStream_t st);
-    cudaError_t backward(int B, cudaStream_t st);
+    cudaError_t infer(const RowSource &r, int B, float *logits, int *classes, cudaStream_t st);
+    cudaError_t gradients(const RowSource &r, int B, float *logits, double *loss, int *correct, cudaStream_t st);
     cudaError_t update(int B, float lr, float wd, cudaStream_t st);
     cudaError_t flat_grad(int B, cudaStream_t st);
-    cudaError_t argmax(int B, int *out, cudaStream_t st);
 };
 
 }  // namespace amrgpu

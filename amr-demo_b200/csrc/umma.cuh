@@ -3,13 +3,14 @@
 // descriptors, the kind::f16 instruction descriptor, tcgen05.mma issue and
 // commit, and TMEM -> register loads. Inline PTX only.
 //
-// Operand layout used throughout (K-major, no swizzle): a tile of R rows x
-// KC elements (bf16) is stored as 8x8 "core matrices" of 128 contiguous
-// bytes (8 rows x 16 bytes); core (r8, k8) sits at byte
-// (r8 * (KC/8) + k8) * 128. In descriptor terms the leading-dimension byte
-// offset (next core matrix along K) is 128 and the stride-dimension byte
-// offset (next group of 8 rows) is KC * 16. One MMA consumes K = 16, i.e.
-// two core matrices along K; the k-th step starts 256 * k bytes further.
+// Operand layouts (no swizzle): a tile is stored as 8x8 "core matrices" of
+// 128 contiguous bytes, 8 rows of 16 bytes. K-major: a row holds 8 K elements
+// of one M (or N) index; the leading-dimension byte offset goes to the next
+// 8 K elements, the stride-dimension byte offset to the next 8 M indices.
+// MN-major: a row holds 8 M (or N) elements of one K index; the leading
+// offset goes to the next 8 K indices, the stride offset to the next 8 M
+// elements. So one row-major copy of a matrix serves as either operand. An
+// MMA consumes K = 16, two core matrices along K.
 #pragma once
 
 #include <cstdint>
@@ -21,7 +22,7 @@ namespace amrgpu {
 // Shared-memory matrix descriptor (sm_100 layout): start address, leading
 // and stride byte offsets (all >> 4), version 1 at bits 46-47, base offset
 // 0, swizzle mode 0 (none) at bits 61-63.
-__device__ __forceinline__ uint64_t umma_desc_kmajor(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes)
+__device__ __forceinline__ uint64_t umma_desc(uint32_t smem_addr, uint32_t lbo_bytes, uint32_t sbo_bytes)
 {
     uint64_t d = 0;
     d |= (uint64_t)((smem_addr >> 4) & 0x3FFFu);
@@ -32,12 +33,14 @@ __device__ __forceinline__ uint64_t umma_desc_kmajor(uint32_t smem_addr, uint32_
 }
 
 // Instruction descriptor of tcgen05.mma kind::f16: D in FP32 (bits 4-5 = 1),
-// A and B in BF16 (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0),
-// N >> 3 at bits 17-22, M >> 4 at bits 24-28.
+// A and B in BF16 (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0;
+// 1 for an MN-major operand), N >> 3 at bits 17-22, M >> 4 at bits 24-28.
 __host__ __device__ constexpr uint32_t umma_idesc_bf16_f32(int M, int N)
 {
     return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
+
+constexpr uint32_t kUmmaMnMajorA = 1u << 15, kUmmaMnMajorB = 1u << 16;
 
 // D[tmem] (+)= A[smem] * B[smem]^T, issued by one thread.
 __device__ __forceinline__ void umma_bf16_ss(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
