@@ -63,9 +63,10 @@ __device__ __forceinline__ void pack_bf16(const float v[16], uint4 out[2])
 }
 
 // Arguments of mlp_tile_kernel. Row b of the batch is row perm[b] (perm null:
-// b) of X and y. Training writes H1, H2, dZ1, dZ2, dL (row-major, B rows) and
-// per 32 rows the loss sum and the correct predictions; logits [B x 16] and
-// classes [B] are written where given.
+// b) of X and y. Training writes H1, H2, dZ1, dZ2, dL (B rows in the weight
+// gradients' order, blocked_index) and per 32 rows the loss sum and the
+// correct predictions; logits [B x 16] and classes [B] are written where
+// given.
 struct TileArgs {
     const bf16 *X;
     const int *perm;
@@ -81,53 +82,65 @@ struct TileArgs {
     int *err;  // error flags (a bounded wait gave up)
 };
 
+// The weights as the tile kernel reads them: K-major core matrices (umma.cuh),
+// all rows of one 16-byte piece after another, so that a run of pieces is one
+// bulk copy. Element (row, k) of an operand of `rows` rows:
+__host__ __device__ constexpr int tiled_index(int rows, int row, int k)
+{
+    return (k / 8) * rows * 8 + row * 8 + k % 8;
+}
+
+// H1, H2, dZ1, dZ2 and dL as mlp_wgrad_kernel reads them: core matrices of 8
+// rows, all 16-byte pieces of 8 rows after another (an MN-major operand's
+// order), so that any run of rows is one bulk copy. Element (row, col), col a
+// multiple of 8, of a matrix of `chunks` pieces a row:
+__device__ __forceinline__ long long blocked_index(int chunks, int row, int col)
+{
+    return ((long long)(row >> 3) * chunks + (col >> 3)) * 64 + (row & 7) * 8;
+}
+
 // Shared memory of mlp_tile_kernel, in bytes. X and W1 fill it until the
-// first GEMM is done; what comes after lives in their place.
+// first GEMM is done; what comes after lives in their place. X's core
+// matrices lie 144 bytes apart along a row, so that neighbouring pieces of a
+// row, copied by neighbouring threads, go to different banks.
 struct TileSmem {
-    static constexpr int x = 0, xw1 = 128 * kFeatIn * 2;
-    static constexpr int w1 = x + xw1;
-    static constexpr int w2 = w1 + xw1, w3 = w2 + kH2 * kH1 * 2;
-    static constexpr int bar = w3 + kOutPad * kH2 * 2;
-    static constexpr int rows = bar + 16;  // row index of each of the 128 rows
+    static constexpr int xpitch = 144, xrows = kFeatIn / 8 * xpitch;  // next piece, next 8 rows
+    static constexpr int x = 0, w1 = x + 16 * xrows;
+    static constexpr int bar = w1 + kH1 * kFeatIn * 2;  // MMA barrier, weight barriers, TMEM address
+    static constexpr int rows = bar + 80;               // row index of each of the 128 rows
     static constexpr int total = rows + 128 * 4;
-    // in X's place
-    static constexpr int h1 = x, t1 = h1 + 128 * kH1 * 2;  // t1: [column][row]
-    static_assert(t1 + 128 * kH1 * 4 <= w1, "H1 and its GELU terms fit where X was");
+    // in X's place; t1: [column][row]
+    static constexpr int h1 = x, t1 = h1 + 128 * kH1 * 2, dl = t1 + 128 * kH1 * 4;
+    static constexpr int w3 = dl + 128 * kOutPad * 2, w3t = w3 + kOutPad * kH2 * 2;
+    static_assert(w3t + kH2 * kOutPad * 2 <= w1, "what follows the first GEMM fits where X was");
     // in W1's place
-    static constexpr int h2 = w1, t2 = h2 + 128 * kH2 * 2;
-    static constexpr int dl = t2 + 128 * kH2 * 4, dz2 = dl + 128 * kOutPad * 2;
-    static constexpr int w2t = dz2 + 128 * kH2 * 2, w3t = w2t + kH1 * kH2 * 2;
-    static_assert(w3t + kH2 * kOutPad * 2 <= w2, "the backward operands fit where W1 was");
+    static constexpr int h2 = w1, t2 = h2 + 128 * kH2 * 2, dz2 = t2 + 128 * kH2 * 4;
+    static constexpr int w2 = dz2 + 128 * kH2 * 2, w2t = w2 + kH2 * kH1 * 2;
+    static_assert(w2t + kH1 * kH2 * 2 <= bar, "and where W1 was");
 };
 
 constexpr int kTileThreads = 512;
 
-// Rows [0, rows) of a K-major operand of `chunks` 16-byte pieces a row,
-// row stride ld elements, into core matrices at dst by cp.async; eight rows
-// of a piece are neighbours, so a warp moves 64 contiguous bytes of eight rows.
-template <int T>
-__device__ __forceinline__ void stage_kmajor(unsigned char *dst, const bf16 *src, int rows, int chunks, int ld)
-{
-    for (int t = threadIdx.x; t < rows * chunks; t += T) {
-        const int r7 = t & 7, c = (t >> 3) % chunks, r8 = (t >> 3) / chunks;
-        cp_async16(dst + (r8 * chunks + c) * 128 + r7 * 16, src + (long long)(8 * r8 + r7) * ld + 8 * c);
-    }
-}
+// A K-major operand in shared memory: where it starts, the bytes to the next
+// 8 K elements and to the next 8 rows.
+struct Operand {
+    uint32_t at, lead, stride;
+};
 
-// D (+)= A B^T over `steps` K = 16 steps, K-major operands of core-matrix
-// rows of `chunks` pieces, from piece c0 on
-__device__ __forceinline__ void issue_kmajor(uint32_t d, const unsigned char *a, const unsigned char *b, int chunks,
-                                             int c0, int steps, uint32_t idesc, bool first)
+// D (+)= A B^T over `steps` K = 16 steps from the operands' K element 8 c0 on
+__device__ __forceinline__ void issue_kmajor(uint32_t d, const Operand &a, const Operand &b, int c0, int steps,
+                                             uint32_t idesc, bool first)
 {
     for (int k = 0; k < steps; ++k) {
-        const uint32_t off = (uint32_t)(c0 + 2 * k) * 128u;
-        umma_bf16_ss(d, umma_desc(smem_u32(a) + off, 128, (uint32_t)chunks * 128u),
-                     umma_desc(smem_u32(b) + off, 128, (uint32_t)chunks * 128u), idesc, (first && k == 0) ? 0u : 1u);
+        const uint32_t c = (uint32_t)(c0 + 2 * k);
+        umma_bf16_ss(d, umma_desc(a.at + c * a.lead, a.lead, a.stride), umma_desc(b.at + c * b.lead, b.lead, b.stride),
+                     idesc, (first && k == 0) ? 0u : 1u);
     }
 }
 
 // One CTA = 128 rows of the batch. 16 warps: warp w reads TMEM lanes (rows)
-// 32 (w % 4) .. and a quarter w / 4 of the columns; thread 0 issues the MMAs.
+// 32 (w % 4) .. and a quarter w / 4 of the columns; thread 0 copies the
+// weights and issues the MMAs.
 template <bool TRAIN>
 __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArgs a)
 {
@@ -135,17 +148,18 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
     constexpr uint32_t kCols = TRAIN ? 512 : 256;
     // accumulators: Z1, Z2 and the logits stay for the backward pass
     constexpr uint32_t dZ1c = 0, dZ2c = 128, dLc = 192, dB2c = 256, dB1c = 320;
-    constexpr int kGroups = 5, kGroupChunks = kFeatIn / 8 / kGroups;
+    constexpr int kGroups = 5, kGroupChunks = kFeatIn / 8 / kGroups, kGroupBytes = kGroupChunks * kH1 * 16;
     extern __shared__ __align__(128) unsigned char sm[];
     uint64_t *bar = reinterpret_cast<uint64_t *>(sm + S::bar);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 1);
+    uint64_t *wbar = bar + 1;  // W1 by groups, W2 and W3, W2^T and W3^T
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 8);
     int *srow = reinterpret_cast<int *>(sm + S::rows);
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int m0 = blockIdx.x * 128;
 
     if (warp == 0) tmem_alloc(tslot, kCols);
     if (tid == 0) {
-        mbar_init(bar, 1);
+        for (int k = 0; k < 8; ++k) mbar_init(bar + k, 1);
         fence_mbar_init();
     }
     stage_launch_gate();
@@ -155,27 +169,27 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
     tc_fence_after();
     const uint32_t tmem = *tslot;
 
-    // ---------------- operands: X and W1 in K groups of 80, then W2 and W3
+    // ---------------- W1 and X in K groups of 80
+    if (tid == 0) {
+        for (int g = 0; g < kGroups; ++g) {
+            mbar_arrive_expect_tx(wbar + g, kGroupBytes);
+            bulk_g2s(sm + S::w1 + g * kGroupBytes, a.W1 + g * (kGroupBytes / 2), kGroupBytes, wbar + g);
+        }
+    }
     for (int g = 0; g < kGroups; ++g) {
         const int c0 = g * kGroupChunks;
-        for (int t = tid; t < 2 * 128 * kGroupChunks; t += kTileThreads) {
-            const bool isx = t < 128 * kGroupChunks;
-            const int u = isx ? t : t - 128 * kGroupChunks;
-            const int r7 = u & 7, c = c0 + (u >> 3) % kGroupChunks, r8 = (u >> 3) / kGroupChunks;
-            const int r = 8 * r8 + r7;
-            unsigned char *dst = sm + (isx ? S::x : S::w1) + (r8 * (kFeatIn / 8) + c) * 128 + r7 * 16;
-            const int row = isx ? srow[r] : r;
-            if (row >= 0) cp_async16(dst, (isx ? a.X : a.W1) + (long long)row * kFeatIn + 8 * c);
+        for (int t = tid; t < 128 * kGroupChunks; t += kTileThreads) {
+            const int r = t / kGroupChunks, c = c0 + t - r * kGroupChunks;
+            unsigned char *dst = sm + S::x + (r >> 3) * S::xrows + c * S::xpitch + (r & 7) * 16;
+            const int row = srow[r];
+            if (row >= 0) cp_async16(dst, a.X + (long long)row * kFeatIn + 8 * c);
             else *reinterpret_cast<uint4 *>(dst) = make_uint4(0u, 0u, 0u, 0u);
         }
         cp_async_commit();
     }
-    stage_kmajor<kTileThreads>(sm + S::w2, a.W2, kH2, kH1 / 8, kH1);
-    stage_kmajor<kTileThreads>(sm + S::w3, a.W3, kOutPad, kH2 / 8, kH2);
-    cp_async_commit();
 
     unsigned phase = 0;
-    int ok = 1;
+    int ok = 1, copies = kGroups;
     // the MMAs issued so far have finished (bounded wait); false ends the block
     auto done = [&]() -> bool {
         if (!mbar_wait_bounded(bar, phase, kWaitLimit)) ok = 0;
@@ -197,36 +211,52 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
         if (tid == 0) atomicOr(a.err, kFlagTimeout);
         cp_async_wait_all();
         mbar_wait_bounded(bar, phase ^ 1u, kWaitLimit);
+        if (tid == 0)
+            for (int k = 0; k < copies; ++k) mbar_wait_bounded(wbar + k, 0, kWaitLimit);
         tc_fence_before();
         __syncthreads();
         if (warp == 0) tmem_dealloc(tmem, kCols);
     };
+    // thread 0: weight copy k has landed
+    auto landed = [&](int k) -> bool {
+        if (!mbar_wait_bounded(wbar + k, 0, kWaitLimit)) ok = 0;
+        return ok != 0;
+    };
+    const uint32_t base = smem_u32(sm);
+    auto tile = [&](int at, int chunks) -> Operand { return {base + (uint32_t)at, 128u, (uint32_t)chunks * 128u}; };
+    auto weights = [&](int at, int rows) -> Operand { return {base + (uint32_t)at, (uint32_t)rows * 16u, 128u}; };
 
     // ---------------- Z1 = X W1^T
     auto group = [&](int g) {
         publish();
-        if (tid == 0)
-            issue_kmajor(tmem + dZ1c, sm + S::x, sm + S::w1, kFeatIn / 8, g * kGroupChunks, kGroupChunks / 2,
-                         umma_idesc_bf16_f32(128, kH1), g == 0);
+        if (tid == 0 && landed(g))
+            issue_kmajor(tmem + dZ1c, Operand{base + S::x, S::xpitch, S::xrows}, weights(S::w1, kH1), g * kGroupChunks,
+                         kGroupChunks / 2, umma_idesc_bf16_f32(128, kH1), g == 0);
     };
-    cp_async_wait_group<5>();
-    group(0);
     cp_async_wait_group<4>();
-    group(1);
+    group(0);
     cp_async_wait_group<3>();
-    group(2);
+    group(1);
     cp_async_wait_group<2>();
-    group(3);
+    group(2);
     cp_async_wait_group<1>();
+    group(3);
+    cp_async_wait_group<0>();
     group(4);
     if (tid == 0) umma_commit(bar);
     if (!done()) return give_up();
-    // the backward operands into W1's place, while H1 is made
-    if (TRAIN) {
-        stage_kmajor<kTileThreads>(sm + S::w2t, a.W2T, kH1, kH2 / 8, kH2);
-        stage_kmajor<kTileThreads>(sm + S::w3t, a.W3T, kH2, kOutPad / 8, kOutPad);
+    // the other weights into X's and W1's place, while H1 is made
+    if (tid == 0) {
+        mbar_arrive_expect_tx(wbar + 5, (kH2 * kH1 + kOutPad * kH2) * 2);
+        bulk_g2s(sm + S::w2, a.W2, kH2 * kH1 * 2, wbar + 5);
+        bulk_g2s(sm + S::w3, a.W3, kOutPad * kH2 * 2, wbar + 5);
+        if (TRAIN) {
+            mbar_arrive_expect_tx(wbar + 6, (kH2 * kH1 + kOutPad * kH2) * 2);
+            bulk_g2s(sm + S::w2t, a.W2T, kH2 * kH1 * 2, wbar + 6);
+            bulk_g2s(sm + S::w3t, a.W3T, kOutPad * kH2 * 2, wbar + 6);
+        }
     }
-    cp_async_commit();
+    copies = TRAIN ? 7 : 6;
 
     const int r = 32 * (warp & 3) + lane, cg = warp >> 2;
     const int row = m0 + r;
@@ -235,7 +265,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
     float *t1 = reinterpret_cast<float *>(sm + S::t1), *t2 = reinterpret_cast<float *>(sm + S::t2);
     // 16 columns from nb on of a hidden layer: + bias, GELU, the next GEMM's
     // operand (and its copy for the weight gradients)
-    auto hidden = [&](uint32_t dcol, const float *bias, int nb, int width, unsigned char *tile, float *tt, bf16 *out) {
+    auto hidden = [&](uint32_t dcol, const float *bias, int nb, int width, int at, float *tt, bf16 *out) {
         float v[16];
         tmem_ld16(tl + dcol + (uint32_t)nb, v);
 #pragma unroll
@@ -247,32 +277,34 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
         }
         uint4 h[2];
         pack_bf16(v, h);
-        unsigned char *dst = tile + ((r >> 3) * (width / 8) + nb / 8) * 128 + (r & 7) * 16;
+        unsigned char *dst = sm + at + ((r >> 3) * (width / 8) + nb / 8) * 128 + (r & 7) * 16;
         *reinterpret_cast<uint4 *>(dst) = h[0];
         *reinterpret_cast<uint4 *>(dst + 128) = h[1];
         if (TRAIN && rv) {
-            uint4 *o = reinterpret_cast<uint4 *>(out + (long long)row * width + nb);
+            uint4 *o = reinterpret_cast<uint4 *>(out + blocked_index(width / 8, row, nb));
             o[0] = h[0];
-            o[1] = h[1];
+            o[8] = h[1];
         }
     };
 #pragma unroll 1
-    for (int nb = 32 * cg; nb < 32 * cg + 32; nb += 16) hidden(dZ1c, a.b1, nb, kH1, sm + S::h1, t1, a.H1);
+    for (int nb = 32 * cg; nb < 32 * cg + 32; nb += 16) hidden(dZ1c, a.b1, nb, kH1, S::h1, t1, a.H1);
 
     // ---------------- Z2 = H1 W2^T
-    cp_async_wait_group<1>();  // W2 and W3 (the backward operands may be under way)
     publish();
     if (tid == 0) {
-        issue_kmajor(tmem + dZ2c, sm + S::h1, sm + S::w2, kH1 / 8, 0, kH1 / 16, umma_idesc_bf16_f32(128, kH2), true);
+        if (landed(5))
+            issue_kmajor(tmem + dZ2c, tile(S::h1, kH1 / 8), weights(S::w2, kH2), 0, kH1 / 16,
+                         umma_idesc_bf16_f32(128, kH2), true);
         umma_commit(bar);
     }
     if (!done()) return give_up();
-    hidden(dZ2c, a.b2, 16 * cg, kH2, sm + S::h2, t2, a.H2);
+    hidden(dZ2c, a.b2, 16 * cg, kH2, S::h2, t2, a.H2);
 
     // ---------------- L = H2 W3^T
     publish();
     if (tid == 0) {
-        issue_kmajor(tmem + dLc, sm + S::h2, sm + S::w3, kH2 / 8, 0, kH2 / 16, umma_idesc_bf16_f32(128, kOutPad), true);
+        issue_kmajor(tmem + dLc, tile(S::h2, kH2 / 8), weights(S::w3, kOutPad), 0, kH2 / 16,
+                     umma_idesc_bf16_f32(128, kOutPad), true);
         umma_commit(bar);
     }
     if (!done()) return give_up();
@@ -313,9 +345,9 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
             *reinterpret_cast<uint4 *>(dst) = h[0];
             *reinterpret_cast<uint4 *>(dst + 128) = h[1];
             if (rv) {
-                uint4 *o = reinterpret_cast<uint4 *>(a.dL + (long long)row * kOutPad);
+                uint4 *o = reinterpret_cast<uint4 *>(a.dL + blocked_index(kOutPad / 8, row, 0));
                 o[0] = h[0];
-                o[1] = h[1];
+                o[8] = h[1];
             }
             loss = warp_sum(loss);
             corr = __reduce_add_sync(0xffffffffu, corr);
@@ -327,15 +359,16 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
     }
     if (TRAIN) {
         // ---------------- dZ2 = (dL W3) * gelu'(Z2)
-        cp_async_wait_all();
         publish();
         if (tid == 0) {
-            issue_kmajor(tmem + dB2c, sm + S::dl, sm + S::w3t, kOutPad / 8, 0, 1, umma_idesc_bf16_f32(128, kH2), true);
+            if (landed(6))
+                issue_kmajor(tmem + dB2c, tile(S::dl, kOutPad / 8), weights(S::w3t, kH2), 0, 1,
+                             umma_idesc_bf16_f32(128, kH2), true);
             umma_commit(bar);
         }
         if (!done()) return give_up();
         // 16 columns from nb on of a hidden layer's gradient
-        auto back = [&](uint32_t dcol, uint32_t zcol, const float *bias, int nb, int width, unsigned char *tile,
+        auto back = [&](uint32_t dcol, uint32_t zcol, const float *bias, int nb, int width, int at,
                         const float *tt, bf16 *out) {
             float v[16], z[16];
             tmem_ld16(tl + dcol + (uint32_t)nb, v);
@@ -344,28 +377,28 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
             for (int k = 0; k < 16; ++k) v[k] *= gelu_grad_f(z[k] + bias[nb + k], tt[(nb + k) * 128 + r]);
             uint4 h[2];
             pack_bf16(v, h);
-            if (tile) {
-                unsigned char *dst = tile + ((r >> 3) * (width / 8) + nb / 8) * 128 + (r & 7) * 16;
+            if (at >= 0) {
+                unsigned char *dst = sm + at + ((r >> 3) * (width / 8) + nb / 8) * 128 + (r & 7) * 16;
                 *reinterpret_cast<uint4 *>(dst) = h[0];
                 *reinterpret_cast<uint4 *>(dst + 128) = h[1];
             }
             if (rv) {
-                uint4 *o = reinterpret_cast<uint4 *>(out + (long long)row * width + nb);
+                uint4 *o = reinterpret_cast<uint4 *>(out + blocked_index(width / 8, row, nb));
                 o[0] = h[0];
-                o[1] = h[1];
+                o[8] = h[1];
             }
         };
-        back(dB2c, dZ2c, a.b2, 16 * cg, kH2, sm + S::dz2, t2, a.dZ2);
+        back(dB2c, dZ2c, a.b2, 16 * cg, kH2, S::dz2, t2, a.dZ2);
         // ---------------- dZ1 = (dZ2 W2) * gelu'(Z1)
         publish();
         if (tid == 0) {
-            issue_kmajor(tmem + dB1c, sm + S::dz2, sm + S::w2t, kH2 / 8, 0, kH2 / 16, umma_idesc_bf16_f32(128, kH1),
-                         true);
+            issue_kmajor(tmem + dB1c, tile(S::dz2, kH2 / 8), weights(S::w2t, kH1), 0, kH2 / 16,
+                         umma_idesc_bf16_f32(128, kH1), true);
             umma_commit(bar);
         }
         if (!done()) return give_up();
 #pragma unroll 1
-        for (int nb = 32 * cg; nb < 32 * cg + 32; nb += 16) back(dB1c, dZ1c, a.b1, nb, kH1, nullptr, t1, a.dZ1);
+        for (int nb = 32 * cg; nb < 32 * cg + 32; nb += 16) back(dB1c, dZ1c, a.b1, nb, kH1, -1, t1, a.dZ1);
     }
     tc_fence_before();
     __syncthreads();
@@ -389,33 +422,35 @@ constexpr int kWgradN1 = kFeatIn / 5;     // columns of a dW1 role
 constexpr int kBiasBlocks = (kH1 + kH2 + kOutPad) / 8;
 constexpr int kBiasRows = 4096;           // rows staged at a time
 constexpr int kWgradA = kWgradK * 128 * 2, kWgradB = kWgradK * kWgradN1 * 2;
-constexpr int kWgradSmem = kWgradA + kWgradB + 16;
+constexpr int kWgradSmem = kWgradA + kWgradB + 48;
 static_assert(kBiasRows * 16 + 32 * 8 * 4 <= kWgradA + kWgradB, "bias rows fit the operands' space");
 
 // The weight gradients' partial sums: one CTA per 256 rows and role, C[M x N]
-// = A^T B with A [256 x M] and B [256 x N] row-major, i.e. both operands
-// MN-major: a core matrix is 8 rows of 16 bytes along M (or N), the leading
-// offset goes to the next 8 rows, the stride offset to the next 16 bytes. The
-// last kBiasBlocks CTAs sum 8 columns each of dZ1, dZ2, dL over the whole
-// batch, each row in lane b % 32's sum, then the lanes as a shuffle tree does.
+// = A^T B with both operands MN-major: the leading offset goes to the next 8
+// rows, the stride offset to the next 16 bytes of a row. Bulk copies bring
+// what the tile kernel wrote, cp.async gathers X's columns (with cp.async for
+// both, the copies took 8 of 12 us). The last kBiasBlocks CTAs sum 8 columns
+// each of dZ1, dZ2, dL over the whole batch, each row in lane b % 32's sum,
+// then the lanes as a shuffle tree does.
 __global__ void __launch_bounds__(kWgradThreads, 2) mlp_wgrad_kernel(const WgradArgs a)
 {
     extern __shared__ __align__(128) unsigned char sm[];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int splits = (a.B + kWgradK - 1) / kWgradK;
-    stage_launch_gate();
     if ((int)blockIdx.x >= splits * kWgradRoles) {
+        stage_launch_gate();
         const int u0 = 8 * ((int)blockIdx.x - splits * kWgradRoles);
         const bf16 *src;
-        int ld;
-        if (u0 < kH1) { src = a.dZ1 + u0; ld = kH1; }
-        else if (u0 < kH1 + kH2) { src = a.dZ2 + (u0 - kH1); ld = kH2; }
-        else { src = a.dL + (u0 - kH1 - kH2); ld = kOutPad; }
+        int chunks, col;
+        if (u0 < kH1) { src = a.dZ1; chunks = kH1 / 8; col = u0; }
+        else if (u0 < kH1 + kH2) { src = a.dZ2; chunks = kH2 / 8; col = u0 - kH1; }
+        else { src = a.dL; chunks = kOutPad / 8; col = u0 - kH1 - kH2; }
         const int u = tid & 7, l = tid >> 3;
         float s = 0.0f;
         for (int b0 = 0; b0 < a.B; b0 += kBiasRows) {
             const int nb = min(kBiasRows, a.B - b0);
-            for (int k = tid; k < nb; k += kWgradThreads) cp_async16(sm + k * 16, src + (long long)(b0 + k) * ld);
+            for (int k = tid; k < nb; k += kWgradThreads)
+                cp_async16(sm + k * 16, src + blocked_index(chunks, b0 + k, col));
             cp_async_commit();
             cp_async_wait_all();
             __syncthreads();
@@ -436,55 +471,65 @@ __global__ void __launch_bounds__(kWgradThreads, 2) mlp_wgrad_kernel(const Wgrad
 
     constexpr uint32_t kCols = 128;
     uint64_t *bar = reinterpret_cast<uint64_t *>(sm + kWgradA + kWgradB);
-    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 1);
+    uint64_t *cbar = bar + 1;  // the bulk copies of each group of 64 rows
+    uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 5);
     const int z = blockIdx.x / kWgradRoles, role = blockIdx.x % kWgradRoles;
     const int k0 = z * kWgradK, kc = min(kWgradK, a.B - k0), kr = (kc + 15) / 16 * 16;
-    // M, N in 16-byte pieces, the operands' rows and where the result goes
-    const int ma = role < 6 ? 16 : 8, nb = role < 5 ? kWgradN1 / 8 : role == 5 ? kH2 / 8 : kOutPad / 8;
+    // A and B in 16-byte pieces a row; dW3 has 64 rows: the other half of the
+    // tile multiplies what follows in shared memory and is not stored
+    const int ma = role < 6 ? kH1 / 8 : kH2 / 8, nb = role < 5 ? kWgradN1 / 8 : role == 5 ? kH2 / 8 : kOutPad / 8;
     const bf16 *A = role < 5 ? a.dZ1 : role == 5 ? a.H1 : a.H2;
-    const bf16 *Bm = role < 5 ? a.X + role * kWgradN1 : role == 5 ? a.dZ2 : a.dL;
-    const int ldb = role < 5 ? kFeatIn : role == 5 ? kH2 : kOutPad;
+    const bf16 *Bm = role == 5 ? a.dZ2 : a.dL;
     if (warp == 0) tmem_alloc(tslot, kCols);
     if (tid == 0) {
-        mbar_init(bar, 1);
+        for (int k = 0; k < 5; ++k) mbar_init(bar + k, 1);
         fence_mbar_init();
     }
+    stage_launch_gate();
     unsigned char *sA = sm, *sB = sm + kWgradA;
-    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-    // rows in four groups, each its own copy group
-    for (int g = 0; g < 4; ++g) {
-        const int ke = min(kr, 64 * (g + 1));
-        for (int t = tid; t < 64 * 16; t += kWgradThreads) {
-            const int k = 64 * g + (t & 7) + 8 * (t >> 7), c = (t >> 3) & 15;
-            if (k >= ke) continue;
-            unsigned char *dst = sA + ((k >> 3) * 16 + c) * 128 + (k & 7) * 16;
-            if (k < kc && c < ma) cp_async16(dst, A + (long long)(k0 + k) * (8 * ma) + 8 * c);
-            else *reinterpret_cast<uint4 *>(dst) = zero;
+    if (tid == 0) {
+        for (int g = 0; 64 * g < kc; ++g) {
+            const int rows = min(64, kc - 64 * g), na = rows * ma * 16, nbytes = role < 5 ? 0 : rows * nb * 16;
+            mbar_arrive_expect_tx(cbar + g, (unsigned)(na + nbytes));
+            bulk_g2s(sA + 64 * g * ma * 16, A + (long long)(k0 + 64 * g) * ma * 8, (unsigned)na, cbar + g);
+            if (nbytes)
+                bulk_g2s(sB + 64 * g * nb * 16, Bm + (long long)(k0 + 64 * g) * nb * 8, (unsigned)nbytes, cbar + g);
         }
-        for (int t = tid; t < 64 * nb; t += kWgradThreads) {
-            const int k = 64 * g + (t & 7) + 8 * ((t >> 3) / nb), c = (t >> 3) % nb;
-            if (k >= ke) continue;
-            unsigned char *dst = sB + ((k >> 3) * nb + c) * 128 + (k & 7) * 16;
-            if (k < kc) {
-                const int row = role < 5 && a.perm ? a.perm[k0 + k] : k0 + k;
-                cp_async16(dst, Bm + (long long)row * ldb + 8 * c);
-            } else {
-                *reinterpret_cast<uint4 *>(dst) = zero;
+    }
+    // rows past the batch, up to a whole K step, are zero
+    for (int t = tid; t < (kr - kc) * (ma + nb); t += kWgradThreads) {
+        const int k = kc + t / (ma + nb), c = t % (ma + nb);
+        unsigned char *dst = c < ma ? sA + ((k >> 3) * ma + c) * 128 : sB + ((k >> 3) * nb + c - ma) * 128;
+        *reinterpret_cast<uint4 *>(dst + (k & 7) * 16) = make_uint4(0u, 0u, 0u, 0u);
+    }
+    // X's columns of the role, in the same four groups; neighbouring threads
+    // take the two halves of a 32-byte sector, then the next row
+    for (int g = 0; g < 4; ++g) {
+        if (role < 5) {
+            constexpr int np = kWgradN1 / 16;
+            for (int t = tid; t < 64 * kWgradN1 / 8; t += kWgradThreads) {
+                const int k = 64 * g + (t >> 1 & 7) + 8 * ((t >> 4) / np), c = (t & 1) + 2 * ((t >> 4) % np);
+                if (k >= kc) continue;
+                const int row = a.perm ? a.perm[k0 + k] : k0 + k;
+                cp_async16(sB + ((k >> 3) * (kWgradN1 / 8) + c) * 128 + (k & 7) * 16,
+                           a.X + (long long)row * kFeatIn + role * kWgradN1 + 8 * c);
             }
         }
         cp_async_commit();
     }
     const uint32_t idesc = umma_idesc_bf16_f32(128, 8 * nb) | kUmmaMnMajorA | kUmmaMnMajorB;
     uint32_t tmem = 0;
+    int ok = 1;
     auto group = [&](int g) {
         fence_async_smem();
         tc_fence_before();
         __syncthreads();
         tc_fence_after();
         tmem = *tslot;
-        if (tid == 0) {
-            for (int k = 64 * g; k < min(kr, 64 * (g + 1)); k += 16)
-                umma_bf16_ss(tmem, umma_desc(smem_u32(sA) + (uint32_t)(k >> 3) * 2048u, 2048, 128),
+        if (tid == 0 && 64 * g < kc) {
+            if (!mbar_wait_bounded(cbar + g, 0, kWaitLimit)) ok = 0;
+            for (int k = 64 * g; ok && k < min(kr, 64 * (g + 1)); k += 16)
+                umma_bf16_ss(tmem, umma_desc(smem_u32(sA) + (uint32_t)((k >> 3) * ma) * 128u, (uint32_t)ma * 128u, 128),
                              umma_desc(smem_u32(sB) + (uint32_t)((k >> 3) * nb) * 128u, (uint32_t)nb * 128u, 128),
                              idesc, k > 0 ? 1u : 0u);
         }
@@ -498,11 +543,15 @@ __global__ void __launch_bounds__(kWgradThreads, 2) mlp_wgrad_kernel(const Wgrad
     cp_async_wait_group<0>();
     group(3);
     if (tid == 0) umma_commit(bar);
-    int ok = mbar_wait_bounded(bar, 0, kWaitLimit) ? 1 : 0;
+    if (!mbar_wait_bounded(bar, 0, kWaitLimit)) ok = 0;
     ok = __syncthreads_and(ok);
     tc_fence_after();
     if (!ok) {
-        if (tid == 0) atomicOr(a.err, kFlagTimeout);
+        // report; the copies and MMAs in flight get another bounded wait
+        if (tid == 0) {
+            atomicOr(a.err, kFlagTimeout);
+            for (int g = 0; 64 * g < kc; ++g) mbar_wait_bounded(cbar + g, 0, kWaitLimit);
+        }
         mbar_wait_bounded(bar, 0, kWaitLimit);
     } else {
         const int row = 32 * (warp & 3) + lane;
@@ -719,14 +768,14 @@ __device__ __forceinline__ float grad_of(const GradArgs &g, int idx)
         return g.gb[kH1 + kH2 + idx - kOffB3] * g.inv_b;
     }
     float s = 0.0f;
-#pragma unroll 8
+#pragma unroll 16
     for (int k = 0; k < g.splits; ++k) s += p[(long long)k * step];
     return s * g.inv_b;
 }
 
 // AdamW (decoupled weight decay, on weights only) on the FP32 master
-// parameters; refreshes the BF16 copies W (row-major) and W^T and the padded
-// FP32 b3 that the tile kernel reads.
+// parameters; refreshes the BF16 copies of W and W^T (tiled_index) and the
+// padded FP32 b3 that the tile kernel reads.
 struct AdamArgs {
     GradArgs g;
     float *w, *m, *v;
@@ -741,26 +790,27 @@ __global__ void __launch_bounds__(256) mlp_adamw_kernel(const AdamArgs a)
     const int idx = blockIdx.x * blockDim.x + threadIdx.x;
     if (idx >= kMlpParams) return;
     const bool weight = idx < kOffB1 || (idx >= kOffW2 && idx < kOffB2) || (idx >= kOffW3 && idx < kOffB3);
+    const float m0 = a.m[idx], v0 = a.v[idx];
+    float w = a.w[idx];
     const float g = grad_of(a.g, idx);
-    const float m = a.b1 * a.m[idx] + (1.0f - a.b1) * g;
-    const float v = a.b2 * a.v[idx] + (1.0f - a.b2) * g * g;
+    const float m = a.b1 * m0 + (1.0f - a.b1) * g;
+    const float v = a.b2 * v0 + (1.0f - a.b2) * g * g;
     a.m[idx] = m;
     a.v[idx] = v;
-    float w = a.w[idx];
     const float wd = weight ? a.wd : 0.0f;
     w -= a.lr * ((m * a.c1) / (sqrtf(v * a.c2) + a.eps) + wd * w);
     a.w[idx] = w;
     const bf16 wb = __float2bfloat16_rn(w);
     if (idx < kOffB1) {
-        a.W1[idx] = wb;
+        a.W1[tiled_index(kH1, idx / kFeatIn, idx % kFeatIn)] = wb;
     } else if (idx >= kOffW2 && idx < kOffB2) {
         const int k = idx - kOffW2, o = k / kH1, i = k % kH1;
-        a.W2[k] = wb;
-        a.W2T[i * kH2 + o] = wb;
+        a.W2[tiled_index(kH2, o, i)] = wb;
+        a.W2T[tiled_index(kH1, i, o)] = wb;
     } else if (idx >= kOffW3 && idx < kOffB3) {
         const int k = idx - kOffW3, o = k / kH2, i = k % kH2;
-        a.W3[k] = wb;
-        a.W3T[i * kOutPad + o] = wb;
+        a.W3[tiled_index(kOutPad, o, i)] = wb;
+        a.W3T[tiled_index(kH2, i, o)] = wb;
     } else if (idx >= kOffB3) {
         a.b3p[idx - kOffB3] = w;
     }
@@ -916,18 +966,19 @@ bool MlpState::refresh_bf16()
     std::vector<bf> w1(size_t(kH1) * kFeatIn), w2(size_t(kH2) * kH1), w3(size_t(kOutPad) * kH2, zero),
         w2t(size_t(kH1) * kH2), w3t(size_t(kH2) * kOutPad, zero);
     std::vector<float> b3(kOutPad, 0.0f);
-    for (int k = 0; k < kH1 * kFeatIn; ++k) w1[size_t(k)] = __float2bfloat16(h[size_t(kParamOff[0] + k)]);
+    for (int k = 0; k < kH1 * kFeatIn; ++k)
+        w1[size_t(tiled_index(kH1, k / kFeatIn, k % kFeatIn))] = __float2bfloat16(h[size_t(kParamOff[0] + k)]);
     for (int o = 0; o < kH2; ++o)
         for (int i = 0; i < kH1; ++i) {
             const bf b = __float2bfloat16(h[size_t(kParamOff[2] + o * kH1 + i)]);
-            w2[size_t(o * kH1 + i)] = b;
-            w2t[size_t(i * kH2 + o)] = b;
+            w2[size_t(tiled_index(kH2, o, i))] = b;
+            w2t[size_t(tiled_index(kH1, i, o))] = b;
         }
     for (int o = 0; o < kOut; ++o) {
         for (int i = 0; i < kH2; ++i) {
             const bf b = __float2bfloat16(h[size_t(kParamOff[4] + o * kH2 + i)]);
-            w3[size_t(o * kH2 + i)] = b;
-            w3t[size_t(i * kOutPad + o)] = b;
+            w3[size_t(tiled_index(kOutPad, o, i))] = b;
+            w3t[size_t(tiled_index(kH2, i, o))] = b;
         }
         b3[size_t(o)] = h[size_t(kParamOff[5] + o)];
     }

@@ -42,7 +42,8 @@ struct MlpState {
     // FP32 master parameters and AdamW moments (flat: W1, b1, W2, b2, W3, b3)
     float *w = nullptr, *m = nullptr, *v = nullptr;
     // BF16 GEMM operands: W1[128x400], W2[64x128], W3[16x64] (rows 3.. zero),
-    // W2^T[128x64], W3^T[64x16]; padded FP32 b3[16]
+    // W2^T[128x64], W3^T[64x16], in the tile kernel's order (tiled_index in
+    // mlp.cu); padded FP32 b3[16]
     __nv_bfloat16 *W1 = nullptr, *W2 = nullptr, *W3 = nullptr, *W2T = nullptr, *W3T = nullptr;
     float *b3p = nullptr;
     int *err = nullptr;
