@@ -23,8 +23,8 @@
 // tensor cores. One kernel per GEMM, with operands staged chunk by chunk and
 // transposed copies for the second operand's layout, took 21 launches and
 // 283 us a batch; a tile that stays in shared and tensor memory, and
-// operands read K-major or MN-major from the same row-major copy, take
-// @@TRAIN@@.
+// operands read K-major or MN-major from the same core matrices, take three
+// launches and 41 us (16 + 10 + 6 and the waits between them).
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -76,6 +76,7 @@ struct TileArgs {
     const float *b1, *b2, *b3;
     float *logits;
     int *cls;
+    int *counts;  // the judge's counts, set to zero (or null)
     bf16 *H1, *H2, *dZ1, *dZ2, *dL;
     double *loss;
     int *correct;
@@ -163,6 +164,7 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
         fence_mbar_init();
     }
     stage_launch_gate();
+    if (!TRAIN && a.counts && blockIdx.x == 0 && tid < 4) a.counts[tid] = 0;
     if (tid < 128) srow[tid] = m0 + tid < a.B ? (a.perm ? a.perm[m0 + tid] : m0 + tid) : -1;
     tc_fence_before();
     __syncthreads();
@@ -176,17 +178,30 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
             bulk_g2s(sm + S::w1 + g * kGroupBytes, a.W1 + g * (kGroupBytes / 2), kGroupBytes, wbar + g);
         }
     }
-    for (int g = 0; g < kGroups; ++g) {
-        const int c0 = g * kGroupChunks;
-        for (int t = tid; t < 128 * kGroupChunks; t += kTileThreads) {
-            const int r = t / kGroupChunks, c = c0 + t - r * kGroupChunks;
-            unsigned char *dst = sm + S::x + (r >> 3) * S::xrows + c * S::xpitch + (r & 7) * 16;
-            const int row = srow[r];
-            if (row >= 0) cp_async16(dst, a.X + (long long)row * kFeatIn + 8 * c);
-            else *reinterpret_cast<uint4 *>(dst) = make_uint4(0u, 0u, 0u, 0u);
+    constexpr int kLoads = (128 * kGroupChunks + kTileThreads - 1) / kTileThreads;
+    uint4 xv[kGroups][kLoads];
+#pragma unroll
+    for (int g = 0; g < kGroups; ++g)
+#pragma unroll
+        for (int u = 0; u < kLoads; ++u) {
+            const int t = tid + u * kTileThreads;
+            xv[g][u] = make_uint4(0u, 0u, 0u, 0u);
+            if (t < 128 * kGroupChunks) {
+                const int r = t / kGroupChunks, c = g * kGroupChunks + t - r * kGroupChunks;
+                const int row = srow[r];
+                if (row >= 0) xv[g][u] = __ldg(reinterpret_cast<const uint4 *>(a.X + (long long)row * kFeatIn + 8 * c));
+            }
         }
-        cp_async_commit();
-    }
+    auto store_x = [&](int g) {
+#pragma unroll
+        for (int u = 0; u < kLoads; ++u) {
+            const int t = tid + u * kTileThreads;
+            if (t < 128 * kGroupChunks) {
+                const int r = t / kGroupChunks, c = g * kGroupChunks + t - r * kGroupChunks;
+                *reinterpret_cast<uint4 *>(sm + S::x + (r >> 3) * S::xrows + c * S::xpitch + (r & 7) * 16) = xv[g][u];
+            }
+        }
+    };
 
     unsigned phase = 0;
     int ok = 1, copies = kGroups;
@@ -209,7 +224,6 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
         // report, and release the tensor memory without writing results;
         // the MMAs in flight get another bounded wait
         if (tid == 0) atomicOr(a.err, kFlagTimeout);
-        cp_async_wait_all();
         mbar_wait_bounded(bar, phase ^ 1u, kWaitLimit);
         if (tid == 0)
             for (int k = 0; k < copies; ++k) mbar_wait_bounded(wbar + k, 0, kWaitLimit);
@@ -233,15 +247,15 @@ __global__ void __launch_bounds__(kTileThreads, 1) mlp_tile_kernel(const TileArg
             issue_kmajor(tmem + dZ1c, Operand{base + S::x, S::xpitch, S::xrows}, weights(S::w1, kH1), g * kGroupChunks,
                          kGroupChunks / 2, umma_idesc_bf16_f32(128, kH1), g == 0);
     };
-    cp_async_wait_group<4>();
+    store_x(0);
     group(0);
-    cp_async_wait_group<3>();
+    store_x(1);
     group(1);
-    cp_async_wait_group<2>();
+    store_x(2);
     group(2);
-    cp_async_wait_group<1>();
+    store_x(3);
     group(3);
-    cp_async_wait_group<0>();
+    store_x(4);
     group(4);
     if (tid == 0) umma_commit(bar);
     if (!done()) return give_up();
@@ -422,7 +436,7 @@ constexpr int kWgradN1 = kFeatIn / 5;     // columns of a dW1 role
 constexpr int kBiasBlocks = (kH1 + kH2 + kOutPad) / 8;
 constexpr int kBiasRows = 4096;           // rows staged at a time
 constexpr int kWgradA = kWgradK * 128 * 2, kWgradB = kWgradK * kWgradN1 * 2;
-constexpr int kWgradSmem = kWgradA + kWgradB + 48;
+constexpr int kWgradSmem = kWgradA + kWgradB + 48 + kWgradK * 4;
 static_assert(kBiasRows * 16 + 32 * 8 * 4 <= kWgradA + kWgradB, "bias rows fit the operands' space");
 
 // The weight gradients' partial sums: one CTA per 256 rows and role, C[M x N]
@@ -473,6 +487,7 @@ __global__ void __launch_bounds__(kWgradThreads, 2) mlp_wgrad_kernel(const Wgrad
     uint64_t *bar = reinterpret_cast<uint64_t *>(sm + kWgradA + kWgradB);
     uint64_t *cbar = bar + 1;  // the bulk copies of each group of 64 rows
     uint32_t *tslot = reinterpret_cast<uint32_t *>(bar + 5);
+    int *srow = reinterpret_cast<int *>(bar + 6);  // the rows of X
     const int z = blockIdx.x / kWgradRoles, role = blockIdx.x % kWgradRoles;
     const int k0 = z * kWgradK, kc = min(kWgradK, a.B - k0), kr = (kc + 15) / 16 * 16;
     // A and B in 16-byte pieces a row; dW3 has 64 rows: the other half of the
@@ -496,6 +511,11 @@ __global__ void __launch_bounds__(kWgradThreads, 2) mlp_wgrad_kernel(const Wgrad
                 bulk_g2s(sB + 64 * g * nb * 16, Bm + (long long)(k0 + 64 * g) * nb * 8, (unsigned)nbytes, cbar + g);
         }
     }
+    if (role < 5) {
+        // (one load for all: read where it is used, the copies waited for it)
+        if (tid < kc) srow[tid] = a.perm ? a.perm[k0 + tid] : k0 + tid;
+        __syncthreads();
+    }
     // rows past the batch, up to a whole K step, are zero
     for (int t = tid; t < (kr - kc) * (ma + nb); t += kWgradThreads) {
         const int k = kc + t / (ma + nb), c = t % (ma + nb);
@@ -510,7 +530,7 @@ __global__ void __launch_bounds__(kWgradThreads, 2) mlp_wgrad_kernel(const Wgrad
             for (int t = tid; t < 64 * kWgradN1 / 8; t += kWgradThreads) {
                 const int k = 64 * g + (t >> 1 & 7) + 8 * ((t >> 4) / np), c = (t & 1) + 2 * ((t >> 4) % np);
                 if (k >= kc) continue;
-                const int row = a.perm ? a.perm[k0 + k] : k0 + k;
+                const int row = srow[k];
                 cp_async16(sB + ((k >> 3) * (kWgradN1 / 8) + c) * 128 + (k & 7) * 16,
                            a.X + (long long)row * kFeatIn + role * kWgradN1 + 8 * c);
             }
@@ -588,107 +608,98 @@ __global__ void __launch_bounds__(kWgradThreads, 2) mlp_wgrad_kernel(const Wgrad
 //   x3 = S (rho E - mean rho E) / mean rho E
 // with a the sound speed of the mean state and S = kFeatScale; layout
 // X[q][c*100 + (J+1)*10 + (I+1)], I, J = -1..8.
+//
+// One warp per quad, a patch in shared memory: 64 cells (two a lane) and the
+// 32 ring cells (one a lane). Bound by the latency of a quad's loads and of
+// its divisions and root, which one warp now does once for the quad: a block
+// of four warps and three barriers per quad took 27 us for 6802 quads of 8x8
+// (14 MB read), this takes
+// 12 us.
+constexpr int kFeatWarps = 4;
+
 template <int N>
-__global__ void __launch_bounds__(128) features_kernel(const double *q, long long stride, const QuadDesc *quads,
-                                                      int nquad, bf16 *X)
+__global__ void __launch_bounds__(32 * kFeatWarps) features_kernel(const double *q, long long stride,
+                                                                   const QuadDesc *quads, int nquad, bf16 *X)
 {
     constexpr int R = N / 8;
     constexpr int NN = N * N;
-    __shared__ double P[4][10][10];
-    __shared__ double red[4][4];
-    const int quad = blockIdx.x;
+    __shared__ double sP[kFeatWarps][4][100];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int quad = blockIdx.x * kFeatWarps + w;
     if (quad >= nquad) return;
-    const int t = threadIdx.x;
+    double(*P)[100] = sP[w];
+    const int sd = lane >> 3, M = lane & 7;
+    const SideDesc d = quads[quad].side[sd];
     const double inv = 1.0 / (double)(R * R);
-    if (t < 64) {
-        const int I = t & 7, J = t >> 3;
+    double v[4][2];
 #pragma unroll
-        for (int f = 0; f < 4; ++f) {
+    for (int f = 0; f < 4; ++f)
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const int I = lane & 7, J = (lane >> 3) + 4 * k;
             double s = 0.0;
 #pragma unroll
             for (int dj = 0; dj < R; ++dj)
 #pragma unroll
                 for (int di = 0; di < R; ++di)
                     s += q[f * stride + (long long)quad * NN + (R * J + dj) * N + (R * I + di)];
-            P[f][J + 1][I + 1] = s * inv;
+            v[f][k] = s * inv;
+            P[f][(J + 1) * 10 + I + 1] = v[f][k];
         }
-    } else if (t < 96) {
-        const int sd = (t - 64) >> 3, M = (t - 64) & 7;
-        const SideDesc d = quads[quad].side[sd];
+    {
+        // box mean over the R cells facing this ring cell (own edge cells
+        // for a boundary side are averaged across the edge only)
         const double rinv = 1.0 / (double)R;
+        const int at = sd == 0 ? (M + 1) * 10 : sd == 1 ? (M + 1) * 10 + 9 : sd == 2 ? M + 1 : 90 + M + 1;
+        const bool own = !(d.kind == kSideFull || d.kind == kSideFineHang || d.kind == kSideCoarseHang);
+        const long long b0 = (long long)(own ? quad : d.nbr0) * NN;
 #pragma unroll
         for (int f = 0; f < 4; ++f) {
             double s = 0.0;
+#pragma unroll
             for (int dm = 0; dm < R; ++dm) {
                 const int m = R * M + dm;
-                if (d.kind == kSideFull || d.kind == kSideFineHang) {
-                    s += q[f * stride + (long long)d.nbr0 * NN + facing_cell<N>(sd, m)];
-                } else if (d.kind == kSideCoarseHang) {
-                    s += 0.5 * (q[f * stride + (long long)d.nbr0 * NN + facing_cell<N>(sd, m)] +
-                                q[f * stride + (long long)d.nbr1 * NN + facing_cell<N>(sd, m)]);
-                } else {
-                    const int own = (sd == 0) ? m * N : (sd == 1) ? m * N + N - 1 : (sd == 2) ? m : (N - 1) * N + m;
-                    s += q[f * stride + (long long)quad * NN + own];
-                }
+                const int oc = (sd == 0) ? m * N : (sd == 1) ? m * N + N - 1 : (sd == 2) ? m : (N - 1) * N + m;
+                const int fc = facing_cell<N>(sd, m);
+                double x = q[f * stride + b0 + (own ? oc : fc)];
+                if (d.kind == kSideCoarseHang) x = 0.5 * (x + q[f * stride + (long long)d.nbr1 * NN + fc]);
+                s += x;
             }
-            // box mean over the R cells facing this ring cell (own edge cells
-            // for a boundary side are averaged across the edge only)
-            const double v = s * rinv;
-            if (sd == 0) P[f][M + 1][0] = v;
-            else if (sd == 1) P[f][M + 1][9] = v;
-            else if (sd == 2) P[f][0][M + 1] = v;
-            else P[f][9][M + 1] = v;
+            P[f][at] = s * rinv;
         }
     }
-    __syncthreads();
-    if (t < 4) {
-        const int cj = (t >> 1) ? 9 : 0, ci = (t & 1) ? 9 : 0;
-        const int pj = (t >> 1) ? 8 : 1, pi = (t & 1) ? 8 : 1;
-#pragma unroll
-        for (int f = 0; f < 4; ++f) P[f][cj][ci] = P[f][pj][pi];
-    }
     // means of the 8 x 8 patch, in a fixed order
-    double m4[4] = {0.0, 0.0, 0.0, 0.0};
-    if (t < 64) {
-        const int I = t & 7, J = t >> 3;
+    double m4[4];
 #pragma unroll
-        for (int f = 0; f < 4; ++f) m4[f] = P[f][J + 1][I + 1];
+    for (int f = 0; f < 4; ++f) m4[f] = (warp_sum(v[f][0]) + warp_sum(v[f][1])) / 64.0;
+    __syncwarp();
+    if (lane < 16) {
+        const int f = lane >> 2, cj = lane & 2 ? 9 : 0, ci = lane & 1 ? 9 : 0;
+        P[f][cj * 10 + ci] = P[f][(lane & 2 ? 8 : 1) * 10 + (lane & 1 ? 8 : 1)];
     }
-#pragma unroll
-    for (int f = 0; f < 4; ++f) m4[f] = warp_sum(m4[f]);
-    if ((t & 31) == 0 && t < 64) {
-#pragma unroll
-        for (int f = 0; f < 4; ++f) red[f][t >> 5] = m4[f];
-    }
-    __syncthreads();
-    const double mr = (red[0][0] + red[0][1]) / 64.0;
-    const double mu = (red[1][0] + red[1][1]) / 64.0;
-    const double mv = (red[2][0] + red[2][1]) / 64.0;
-    const double me = (red[3][0] + red[3][1]) / 64.0;
+    const double mr = m4[0], mu = m4[1], mv = m4[2], me = m4[3];
     const double pbar = 0.4 * (me - 0.5 * (mu * mu + mv * mv) / mr);
     const double c2 = 1.4 * pbar / mr;
     const double abar = sqrt(c2 > 1e-24 ? c2 : 1e-24);
     const double sc[4] = {kFeatScale / mr, kFeatScale / (mr * abar), kFeatScale / (mr * abar), kFeatScale / me};
-    const double mm[4] = {mr, mu, mv, me};
-    for (int k = t; k < kFeatIn; k += 128) {
-        const int f = k / 100, r = k % 100;
-        const double x = (P[f][r / 10][r % 10] - mm[f]) * sc[f];
-        X[(long long)quad * kFeatIn + k] = __float2bfloat16_rn((float)x);
-    }
+    __syncwarp();
+    __nv_bfloat162 *out = reinterpret_cast<__nv_bfloat162 *>(X + (long long)quad * kFeatIn);
+#pragma unroll
+    for (int f = 0; f < 4; ++f)
+        for (int k = lane; k < 50; k += 32) {
+            const double x0 = (P[f][2 * k] - m4[f]) * sc[f], x1 = (P[f][2 * k + 1] - m4[f]) * sc[f];
+            out[50 * f + k] = __nv_bfloat162(__float2bfloat16_rn((float)x0), __float2bfloat16_rn((float)x1));
+        }
 }
 
 // Largest relative density jump of a quad (the plain indicator's method 5
 // quantity, as in tag_kernel): between adjacent cells of the patch and
 // between an edge cell and the neighbour cell(s) its face flux pairs it
-// with. Quads listed in `which` (or all when null), one warp each.
+// with. By one warp, whose lanes all get it.
 template <int N>
-__global__ void jump_kernel(const double *rho, const QuadDesc *quads, const int *which, int count, double *jump)
+__device__ __forceinline__ double jump_of(const double *rho, const QuadDesc *quads, int quad, int lane)
 {
     constexpr int NN = N * N;
-    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    if (w >= count) return;
-    const int quad = which ? which[w] : w;
     const double *p = rho + (long long)quad * NN;
     auto rj = [](double x, double y) { return fabs(x - y) / fmin(x, y); };
     double J = 0.0;
@@ -708,19 +719,34 @@ __global__ void jump_kernel(const double *rho, const QuadDesc *quads, const int 
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) J = fmax(J, __shfl_xor_sync(0xffffffffu, J, o));
+    return J;
+}
+
+template <int N>
+__global__ void jump_kernel(const double *rho, const QuadDesc *quads, int nquad, double *jump)
+{
+    const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (w >= nquad) return;
+    const double J = jump_of<N>(rho, quads, w, lane);
     if (lane == 0) jump[w] = J;
 }
 
-// plain three-class label from the jump: refine (1) when J >= tol, coarsen
-// (0) when J < lo_frac * tol, keep (2) in between. cover: merged into the
-// label already there, keeping the finer demand (refine if either asks for
-// it, coarsen only if both do, keep otherwise)
+// plain three-class label of a jump: refine (1) when J >= tol, coarsen (0)
+// when J < lo_frac * tol, keep (2) in between
+__device__ __forceinline__ int class_of(double j, double tol, double lo_frac)
+{
+    return j >= tol ? kClassRefine : (j < lo_frac * tol ? kClassCoarsen : kClassKeep);
+}
+
+// Labels of n jumps. cover: merged into the label already there, keeping the
+// finer demand (refine if either asks for it, coarsen only if both do, keep
+// otherwise)
 __global__ void label_kernel(const double *J, int n, double tol, double lo_frac, int *cls, int cover)
 {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= n) return;
-    const double j = J[k];
-    int c = j >= tol ? kClassRefine : (j < lo_frac * tol ? kClassCoarsen : kClassKeep);
+    int c = class_of(J[k], tol, lo_frac);
     if (cover) {
         const int old = cls[k];
         c = (old == kClassRefine || c == kClassRefine) ? kClassRefine
@@ -729,6 +755,33 @@ __global__ void label_kernel(const double *J, int n, double tol, double lo_frac,
     cls[k] = c;
 }
 
+// The judge: the plain class of the quads that a hash of (seed, quad) puts
+// below `fraction`, against the learned class, one warp per quad. counts[0]:
+// judged, [1]: the classes differ, [2]: the learned one is coarser (the tile
+// kernel has set them to zero). On the host the sampling loop and the two
+// copies of the sample cost 30-40 us at 7000 quads, most of a call.
+template <int N>
+__global__ void __launch_bounds__(256) judge_kernel(const double *rho, const QuadDesc *quads, int nquad,
+                                                    unsigned long long seed, double fraction, double tol,
+                                                    double lo_frac, const int *cls, int *counts)
+{
+    const int quad = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (quad >= nquad) return;
+    unsigned long long z = seed * 0x9E3779B97F4A7C15ull + (unsigned long long)quad * 0xD1B54A32D192ED03ull +
+                           0x8CB92BA72F3D8DD7ull;
+    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
+    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
+    z ^= z >> 31;
+    if (!((double)(z >> 11) * (1.0 / 9007199254740992.0) < fraction)) return;
+    const int p = class_of(jump_of<N>(rho, quads, quad, lane), tol, lo_frac), t = cls[quad];
+    if (lane == 0) {
+        atomicAdd(counts, 1);
+        if (p != t) atomicAdd(counts + 1, 1);
+        if ((p == kClassRefine && t != kClassRefine) || (t == kClassCoarsen && p != kClassCoarsen))
+            atomicAdd(counts + 2, 1);
+    }
+}
 
 // ---------------------------------------------------------------- optimiser
 
@@ -742,6 +795,21 @@ struct GradArgs {
 
 constexpr int kOffB1 = kH1 * kFeatIn, kOffW2 = kOffB1 + kH1, kOffB2 = kOffW2 + kH2 * kH1, kOffW3 = kOffB2 + kH2,
               kOffB3 = kOffW3 + kOut * kH2;
+
+// Thread t's flat parameter: W2 and W3 in the order of their partials, which
+// hold the transposes, so that neighbouring threads read neighbours.
+__device__ __forceinline__ int param_of(int t)
+{
+    if (t >= kOffW2 && t < kOffB2) {
+        const int k = t - kOffW2;
+        return kOffW2 + (k % kH2) * kH1 + k / kH2;
+    }
+    if (t >= kOffW3 && t < kOffB3) {
+        const int k = t - kOffW3;
+        return kOffW3 + (k % kOut) * kH2 + k / kOut;
+    }
+    return t;
+}
 
 // Gradient of flat parameter idx: a weight's is the sum over the partials in
 // order, read transposed where they hold W^T.
@@ -768,7 +836,7 @@ __device__ __forceinline__ float grad_of(const GradArgs &g, int idx)
         return g.gb[kH1 + kH2 + idx - kOffB3] * g.inv_b;
     }
     float s = 0.0f;
-#pragma unroll 16
+#pragma unroll 32
     for (int k = 0; k < g.splits; ++k) s += p[(long long)k * step];
     return s * g.inv_b;
 }
@@ -784,11 +852,12 @@ struct AdamArgs {
     float lr, wd, b1, b2, eps, c1, c2;  // c1 = 1/(1-b1^t), c2 = 1/(1-b2^t)
 };
 
-__global__ void __launch_bounds__(256) mlp_adamw_kernel(const AdamArgs a)
+__global__ void __launch_bounds__(128) mlp_adamw_kernel(const AdamArgs a)
 {
     stage_launch_gate();
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= kMlpParams) return;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= kMlpParams) return;
+    const int idx = param_of(t);
     const bool weight = idx < kOffB1 || (idx >= kOffW2 && idx < kOffB2) || (idx >= kOffW3 && idx < kOffB3);
     const float m0 = a.m[idx], v0 = a.v[idx];
     float w = a.w[idx];
@@ -818,8 +887,10 @@ __global__ void __launch_bounds__(256) mlp_adamw_kernel(const AdamArgs a)
 
 __global__ void __launch_bounds__(256) mlp_grad_kernel(const GradArgs g, float *out)
 {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx < kMlpParams) out[idx] = grad_of(g, idx);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= kMlpParams) return;
+    const int idx = param_of(t);
+    out[idx] = grad_of(g, idx);
 }
 
 // ---------------------------------------------------------------- host side
@@ -828,24 +899,37 @@ cudaError_t mlp_launch_features(int n, const double *q, long long stride, const 
                                 cudaStream_t st)
 {
     if (nquad <= 0) return cudaSuccess;
+    const int blocks = (nquad + kFeatWarps - 1) / kFeatWarps;
     switch (n) {
-    case 8: features_kernel<8><<<nquad, 128, 0, st>>>(q, stride, quads, nquad, X); break;
-    case 16: features_kernel<16><<<nquad, 128, 0, st>>>(q, stride, quads, nquad, X); break;
+    case 8: features_kernel<8><<<blocks, 32 * kFeatWarps, 0, st>>>(q, stride, quads, nquad, X); break;
+    case 16: features_kernel<16><<<blocks, 32 * kFeatWarps, 0, st>>>(q, stride, quads, nquad, X); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 
-cudaError_t mlp_launch_jump(int n, const double *rho, const QuadDesc *quads, const int *which, int count, double *J,
-                            cudaStream_t st)
+cudaError_t mlp_launch_jump(int n, const double *rho, const QuadDesc *quads, int nquad, double *J, cudaStream_t st)
 {
-    if (count <= 0) return cudaSuccess;
-    const int blocks = (count * 32 + 255) / 256;
+    if (nquad <= 0) return cudaSuccess;
+    const int blocks = (nquad * 32 + 255) / 256;
     switch (n) {
-    case 2: jump_kernel<2><<<blocks, 256, 0, st>>>(rho, quads, which, count, J); break;
-    case 4: jump_kernel<4><<<blocks, 256, 0, st>>>(rho, quads, which, count, J); break;
-    case 8: jump_kernel<8><<<blocks, 256, 0, st>>>(rho, quads, which, count, J); break;
-    case 16: jump_kernel<16><<<blocks, 256, 0, st>>>(rho, quads, which, count, J); break;
+    case 2: jump_kernel<2><<<blocks, 256, 0, st>>>(rho, quads, nquad, J); break;
+    case 4: jump_kernel<4><<<blocks, 256, 0, st>>>(rho, quads, nquad, J); break;
+    case 8: jump_kernel<8><<<blocks, 256, 0, st>>>(rho, quads, nquad, J); break;
+    case 16: jump_kernel<16><<<blocks, 256, 0, st>>>(rho, quads, nquad, J); break;
+    default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t mlp_launch_judge(int n, const double *rho, const QuadDesc *quads, int nquad, unsigned long long seed,
+                             double fraction, double tol, double lo_frac, const int *cls, int *counts, cudaStream_t st)
+{
+    if (nquad <= 0) return cudaSuccess;
+    const int blocks = (nquad * 32 + 255) / 256;
+    switch (n) {
+    case 8: judge_kernel<8><<<blocks, 256, 0, st>>>(rho, quads, nquad, seed, fraction, tol, lo_frac, cls, counts); break;
+    case 16: judge_kernel<16><<<blocks, 256, 0, st>>>(rho, quads, nquad, seed, fraction, tol, lo_frac, cls, counts); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
@@ -906,20 +990,19 @@ void MlpState::release()
     cudaFree(yall);
     cudaFree(perm);
     cudaFree(jump);
-    cudaFree(which);
-    cudaFree(jcls);
     cudaFree(stats);
+    cudaFreeHost(h_back);
+    h_back = nullptr;
+    cap_back = 0;
     cap_stats = 0;
     stats = nullptr;
     Xall = nullptr;
     yall = nullptr;
     perm = nullptr;
     jump = nullptr;
-    which = nullptr;
-    jcls = nullptr;
     cap_batch = cap_train = 0;
     cap_data = n_data = cap_perm = 0;
-    cap_judge = 0;
+    cap_jump = 0;
 }
 
 bool MlpState::init(uint64_t seed)
@@ -1008,7 +1091,7 @@ bool MlpState::ensure_batch(int B, bool train)
     auto &o = batch_owned;
     const size_t b = size_t(B);
     const size_t splits = (b + kWgradK - 1) / kWgradK;
-    bool ok = dalloc(&X, b * kFeatIn, o) && dalloc(&y, b, o) && dalloc(&Lg, b * kOutPad, o) && dalloc(&cls, b, o);
+    bool ok = dalloc(&X, b * kFeatIn, o) && dalloc(&y, b, o) && dalloc(&Lg, b * kOutPad, o) && dalloc(&cls, b + 4, o);
     if (ok && train)
         ok = dalloc(&H1, b * kH1, o) && dalloc(&H2, b * kH2, o) && dalloc(&dZ1, b * kH1, o) &&
              dalloc(&dZ2, b * kH2, o) && dalloc(&dL, b * kOutPad, o) && dalloc(&P1, splits * kH1 * kFeatIn, o) &&
@@ -1057,22 +1140,29 @@ bool MlpState::ensure_data(long long n)
     return true;
 }
 
-bool MlpState::ensure_judge(int n)
+bool MlpState::ensure_jump(int n)
 {
-    if (n <= cap_judge) return true;
-    n = std::max(2 * n, 1024);  // headroom: the judged quads follow the mesh
+    if (n <= cap_jump) return true;
+    n = std::max(2 * n, 1024);  // headroom: a mesh that grows reallocates rarely
     cudaStreamSynchronize(stream);
     cudaFree(jump);
-    cudaFree(which);
-    cudaFree(jcls);
     jump = nullptr;
-    which = jcls = nullptr;
-    cap_judge = 0;
-    if (cudaMalloc(&jump, sizeof(double) * size_t(n)) != cudaSuccess ||
-        cudaMalloc(&which, sizeof(int) * size_t(n)) != cudaSuccess ||
-        cudaMalloc(&jcls, sizeof(int) * size_t(n)) != cudaSuccess)
-        return false;
-    cap_judge = n;
+    cap_jump = 0;
+    if (cudaMalloc(&jump, sizeof(double) * size_t(n)) != cudaSuccess) return false;
+    cap_jump = n;
+    return true;
+}
+
+bool MlpState::ensure_back(size_t bytes)
+{
+    if (bytes <= cap_back) return true;
+    cudaStreamSynchronize(stream);
+    cudaFreeHost(h_back);
+    h_back = nullptr;
+    cap_back = 0;
+    bytes = std::max<size_t>(2 * bytes, 4096);
+    if (cudaMallocHost(&h_back, bytes) != cudaSuccess) return false;
+    cap_back = bytes;
     return true;
 }
 
@@ -1120,14 +1210,16 @@ cudaError_t opt_in()
 
 }  // namespace
 
-// Forward pass of B rows: logits [B x 16] and classes where given.
-cudaError_t MlpState::infer(const RowSource &r, int B, float *logits, int *classes, cudaStream_t st)
+// Forward pass of B rows: logits [B x 16] and classes where given; the
+// judge's counts, where given, set to zero.
+cudaError_t MlpState::infer(const RowSource &r, int B, float *logits, int *classes, int *counts, cudaStream_t st)
 {
     cudaError_t e = opt_in();
     if (e != cudaSuccess) return e;
     TileArgs a = tile_args(*this, r, B);
     a.logits = logits;
     a.cls = classes;
+    a.counts = counts;
     return launch_after((const void *)mlp_tile_kernel<false>, (B + 127) / 128, kTileThreads, TileSmem::total, a, st);
 }
 
@@ -1173,7 +1265,7 @@ cudaError_t MlpState::update(int B, float lr, float wd, cudaStream_t st)
     a.eps = 1e-8f;
     a.c1 = (float)(1.0 / (1.0 - std::pow((double)b1, (double)step)));
     a.c2 = (float)(1.0 / (1.0 - std::pow((double)b2, (double)step)));
-    return launch_after((const void *)mlp_adamw_kernel, (kMlpParams + 255) / 256, 256, 0, a, st);
+    return launch_after((const void *)mlp_adamw_kernel, (kMlpParams + 127) / 128, 128, 0, a, st);
 }
 
 cudaError_t MlpState::flat_grad(int B, cudaStream_t st)

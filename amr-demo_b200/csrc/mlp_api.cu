@@ -43,16 +43,6 @@ bool check_flags(MlpState &s)
     return true;
 }
 
-// hash of (seed, quad) in [0, 1): the judge's sample
-double judge_u01(unsigned long long seed, int q)
-{
-    uint64_t z = seed * 0x9E3779B97F4A7C15ULL + (uint64_t)q * 0xD1B54A32D192ED03ULL + 0x8CB92BA72F3D8DD7ULL;
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ULL;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBULL;
-    z ^= z >> 31;
-    return (double)(z >> 11) * (1.0 / 9007199254740992.0);
-}
-
 // total + the losses of one batch, given per 32 rows: 256 rows are summed at
 // a time, then added
 double add_losses(double total, const double *loss, long long groups)
@@ -143,7 +133,7 @@ int amrgpu_session_jumps(amrgpu_session_t *s, double *jumps)
         set_error(AMRGPU_ERR_CUDA, "jumps: scratch allocation failed");
         return AMRGPU_ERR_CUDA;
     }
-    bool ok = ok_cuda(mlp_launch_jump(v.n, v.q, v.quads, nullptr, v.nquad, d, st), "jump kernel") &&
+    bool ok = ok_cuda(mlp_launch_jump(v.n, v.q, v.quads, v.nquad, d, st), "jump kernel") &&
               ok_cuda(cudaMemcpyAsync(jumps, d, sizeof(double) * size_t(v.nquad), cudaMemcpyDeviceToHost, st),
                       "D2H jumps") &&
               ok_cuda(cudaStreamSynchronize(st), "sync");
@@ -162,13 +152,13 @@ long long amrgpu_mlp_dataset_append(amrgpu_mlp_t *m, amrgpu_session_t *s, double
     MlpState &ms = m->st;
     cudaStream_t st = (cudaStream_t)v.stream;
     if (!ok_cuda(cudaStreamSynchronize(ms.stream), "sync")) return AMRGPU_ERR_CUDA;
-    if (!ms.ensure_data(ms.n_data + v.nquad) || !ms.ensure_judge(v.nquad)) {
+    if (!ms.ensure_data(ms.n_data + v.nquad) || !ms.ensure_jump(v.nquad)) {
         set_error(AMRGPU_ERR_CUDA, "dataset: device allocation failed");
         return AMRGPU_ERR_CUDA;
     }
     bool ok = ok_cuda(mlp_launch_features(v.n, v.q, v.stride, v.quads, v.nquad, ms.Xall + ms.n_data * kFeatIn, st),
                       "features kernel") &&
-              ok_cuda(mlp_launch_jump(v.n, v.q, v.quads, nullptr, v.nquad, ms.jump, st), "jump kernel") &&
+              ok_cuda(mlp_launch_jump(v.n, v.q, v.quads, v.nquad, ms.jump, st), "jump kernel") &&
               ok_cuda(mlp_launch_labels(ms.jump, v.nquad, tol, lo_frac, ms.yall + ms.n_data, st), "label kernel") &&
               ok_cuda(cudaStreamSynchronize(st), "sync");
     session_count_launches(s, 3);
@@ -188,9 +178,9 @@ int relabel_rows(amrgpu_mlp_t *m, amrgpu_session_t *s, long long first, double t
         return AMRGPU_ERR_ARG;
     MlpState &ms = m->st;
     cudaStream_t st = (cudaStream_t)v.stream;
-    if (!ms.ensure_judge(v.nquad)) return AMRGPU_ERR_CUDA;
+    if (!ms.ensure_jump(v.nquad)) return AMRGPU_ERR_CUDA;
     bool ok = ok_cuda(cudaStreamSynchronize(ms.stream), "sync") &&
-              ok_cuda(mlp_launch_jump(v.n, v.q, v.quads, nullptr, v.nquad, ms.jump, st), "jump kernel") &&
+              ok_cuda(mlp_launch_jump(v.n, v.q, v.quads, v.nquad, ms.jump, st), "jump kernel") &&
               ok_cuda(mlp_launch_labels(ms.jump, v.nquad, tol, lo_frac, ms.yall + first, st, cover), "label kernel") &&
               ok_cuda(cudaStreamSynchronize(st), "sync");
     session_count_launches(s, 2);
@@ -329,7 +319,7 @@ int amrgpu_mlp_predict(amrgpu_mlp_t *m, const uint16_t *features, int batch, flo
     bool ok = ok_cuda(cudaMemcpyAsync(ms.X, features, sizeof(uint16_t) * size_t(batch) * kFeatIn,
                                       cudaMemcpyHostToDevice, st),
                       "H2D") &&
-              ok_cuda(ms.infer(RowSource{ms.X, nullptr, nullptr}, batch, ms.Lg, nullptr, st), "forward") &&
+              ok_cuda(ms.infer(RowSource{ms.X, nullptr, nullptr}, batch, ms.Lg, nullptr, nullptr, st), "forward") &&
               ok_cuda(cudaMemcpyAsync(lg.data(), ms.Lg, sizeof(float) * lg.size(), cudaMemcpyDeviceToHost, st), "D2H") &&
               ok_cuda(cudaStreamSynchronize(st), "sync") && check_flags(ms);
     if (!ok) return AMRGPU_ERR_CUDA;
@@ -353,43 +343,32 @@ int amrgpu_session_learned_tags(amrgpu_session_t *s, amrgpu_mlp_t *m, double jud
     cudaStream_t st = (cudaStream_t)v.stream;
     if (!ok_cuda(cudaStreamSynchronize(ms.stream), "sync")) return AMRGPU_ERR_CUDA;
     const int B = ((v.nquad + 127) / 128) * 128;
-    if (!ms.ensure_batch(B, false) || !ms.ensure_judge(v.nquad)) {
+    const size_t nq = size_t(v.nquad);
+    if (!ms.ensure_batch(B, false) || !ms.ensure_back(sizeof(int) * (nq + 5))) {
         set_error(AMRGPU_ERR_CUDA, "learned tags: device allocation failed");
         return AMRGPU_ERR_CUDA;
     }
-    // the judge's sample
-    std::vector<int> which;
-    if (judge_fraction > 0.0)
-        for (int q = 0; q < v.nquad; ++q)
-            if (judge_u01(seed, q) < judge_fraction) which.push_back(q);
-    const int nj = int(which.size());
-    std::vector<int> jl((size_t)nj);
+    // the classes, the judge's counts behind them and the wait flags come
+    // back together
+    int *back = static_cast<int *>(ms.h_back), *counts = ms.cls + nq;
+    const bool judged = judge_fraction > 0.0;
     bool ok = ok_cuda(mlp_launch_features(v.n, v.q, v.stride, v.quads, v.nquad, ms.X, st), "features kernel") &&
-              ok_cuda(ms.infer(RowSource{ms.X, nullptr, nullptr}, v.nquad, nullptr, ms.cls, st), "forward") &&
-              ok_cuda(cudaMemcpyAsync(tags, ms.cls, sizeof(int) * size_t(v.nquad), cudaMemcpyDeviceToHost, st), "D2H");
-    int launches = 2;
-    if (ok && nj > 0) {
-        ok = ok_cuda(cudaMemcpyAsync(ms.which, which.data(), sizeof(int) * size_t(nj), cudaMemcpyHostToDevice, st),
-                     "H2D judge") &&
-             ok_cuda(mlp_launch_jump(v.n, v.q, v.quads, ms.which, nj, ms.jump, st), "jump kernel") &&
-             ok_cuda(mlp_launch_labels(ms.jump, nj, tol, lo_frac, ms.jcls, st), "label kernel") &&
-             ok_cuda(cudaMemcpyAsync(jl.data(), ms.jcls, sizeof(int) * size_t(nj), cudaMemcpyDeviceToHost, st), "D2H");
-        launches += 2;
-    }
-    if (ok) ok = ok_cuda(cudaStreamSynchronize(st), "sync") && check_flags(ms);
-    session_count_launches(s, launches);
+              ok_cuda(ms.infer(RowSource{ms.X, nullptr, nullptr}, v.nquad, nullptr, ms.cls, counts, st), "forward");
+    if (ok && judged)
+        ok = ok_cuda(mlp_launch_judge(v.n, v.q, v.quads, v.nquad, seed, judge_fraction, tol, lo_frac, ms.cls, counts, st),
+                     "judge kernel");
+    ok = ok && ok_cuda(cudaMemcpyAsync(back, ms.cls, sizeof(int) * (nq + 4), cudaMemcpyDeviceToHost, st), "D2H") &&
+         ok_cuda(cudaMemcpyAsync(back + nq + 4, ms.err, sizeof(int), cudaMemcpyDeviceToHost, st), "D2H") &&
+         ok_cuda(cudaStreamSynchronize(st), "sync");
+    session_count_launches(s, judged ? 3 : 2);
     if (!ok) return AMRGPU_ERR_CUDA;
+    if (back[nq + 4] && !check_flags(ms)) return AMRGPU_ERR_CUDA;
+    std::memcpy(tags, back, sizeof(int) * nq);
     if (judge) {
-        int dis = 0, coarser = 0;
-        for (int k = 0; k < nj; ++k) {
-            const int p = jl[size_t(k)], t = tags[which[size_t(k)]];
-            dis += p != t;
-            coarser += (p == kClassRefine && t != kClassRefine) || (t == kClassCoarsen && p != kClassCoarsen);
-        }
-        judge->judged = nj;
-        judge->disagree = dis;
-        judge->rate = nj ? (double)dis / nj : 0.0;
-        judge->coarser = coarser;
+        judge->judged = back[nq];
+        judge->disagree = back[nq + 1];
+        judge->rate = back[nq] ? (double)back[nq + 1] / back[nq] : 0.0;
+        judge->coarser = back[nq + 2];
     }
     return AMRGPU_OK;
 }

@@ -26,8 +26,9 @@ enum : int { kClassCoarsen = 0, kClassRefine = 1, kClassKeep = 2 };
 
 cudaError_t mlp_launch_features(int n, const double *q, long long stride, const QuadDesc *quads, int nquad,
                                 __nv_bfloat16 *X, cudaStream_t st);
-cudaError_t mlp_launch_jump(int n, const double *rho, const QuadDesc *quads, const int *which, int count, double *J,
-                            cudaStream_t st);
+cudaError_t mlp_launch_jump(int n, const double *rho, const QuadDesc *quads, int nquad, double *J, cudaStream_t st);
+cudaError_t mlp_launch_judge(int n, const double *rho, const QuadDesc *quads, int nquad, unsigned long long seed,
+                             double fraction, double tol, double lo_frac, const int *cls, int *counts, cudaStream_t st);
 cudaError_t mlp_launch_labels(const double *J, int n, double tol, double lo_frac, int *cls, cudaStream_t st,
                               bool cover = false);
 
@@ -56,7 +57,7 @@ struct MlpState {
     int cap_batch = 0, cap_train = 0;
     __nv_bfloat16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *dL = nullptr, *dZ2 = nullptr, *dZ1 = nullptr;
     float *Lg = nullptr, *P1 = nullptr, *P2 = nullptr, *P3 = nullptr, *gb = nullptr, *gflat = nullptr;
-    int *y = nullptr, *cls = nullptr;
+    int *y = nullptr, *cls = nullptr;  // cls: cap_batch classes, then the judge's counts
     std::vector<void *> batch_owned;
     // per 32 rows of every batch of an epoch: loss sums, then correct
     // predictions (ints), in one allocation
@@ -70,10 +71,10 @@ struct MlpState {
     int *perm = nullptr;
     long long cap_perm = 0;
 
-    // judge / inference scratch
-    double *jump = nullptr;
-    int *which = nullptr, *jcls = nullptr;
-    int cap_judge = 0;
+    double *jump = nullptr;  // jumps of a session's quads
+    int cap_jump = 0;
+    void *h_back = nullptr;  // pinned: classes, the judge's counts and the wait flags come back here
+    size_t cap_back = 0;
 
     cudaStream_t stream = nullptr;
 
@@ -85,8 +86,9 @@ struct MlpState {
     bool ensure_batch(int B, bool train);
     bool ensure_stats(long long groups);
     bool ensure_data(long long n);
-    bool ensure_judge(int n);
-    cudaError_t infer(const RowSource &r, int B, float *logits, int *classes, cudaStream_t st);
+    bool ensure_jump(int n);
+    bool ensure_back(size_t bytes);
+    cudaError_t infer(const RowSource &r, int B, float *logits, int *classes, int *counts, cudaStream_t st);
     cudaError_t gradients(const RowSource &r, int B, float *logits, double *loss, int *correct, cudaStream_t st);
     cudaError_t update(int B, float lr, float wd, cudaStream_t st);
     cudaError_t flat_grad(int B, cudaStream_t st);
