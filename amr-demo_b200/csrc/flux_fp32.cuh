@@ -242,21 +242,21 @@ __device__ __forceinline__ void roe_flux_axis_fp32(const float *L, const float *
     flux[3] = o[3];
 }
 
-// A cell's two interior faces at once in packed pairs: its x-face (low
-// side Lx, normal +x, length hx_face) in the first half and its y-face (low
-// side Ly, normal +y, length hy_face) in the second, both with high side P.
-// Each half carries exactly the bits roe_flux_axis_fp32 gives that face.
-__device__ __forceinline__ void roe_flux_axis_pair_fp32(const float *Lx, const float *Ly, const float *P,
-                                                        float hx_face, float hy_face, float fx[4], float fy[4])
+// Two faces at once in packed pairs: an x-face (sides Lx and Rx, normal +x,
+// length hx) in the first half and a y-face (Ly and Ry, normal +y, length
+// hy) in the second. Each half carries exactly the bits roe_flux_axis_fp32
+// gives that face.
+__device__ __forceinline__ void roe_flux_axis_pair_fp32(const float *Lx, const float *Rx, const float *Ly,
+                                                        const float *Ry, float hx, float hy, float fx[4], float fy[4])
 {
-    const AxisSide<float> lx = axis_side<0>(Lx), ly = axis_side<1>(Ly), rx = axis_side<0>(P), ry = axis_side<1>(P);
+    const AxisSide<float> lx = axis_side<0>(Lx), ly = axis_side<1>(Ly), rx = axis_side<0>(Rx), ry = axis_side<1>(Ry);
     auto pair = [](const AxisSide<float> &a, const AxisSide<float> &b) {
         return AxisSide<float2>{make_float2(a.rho, b.rho), make_float2(a.n, b.n), make_float2(a.t, b.t),
                                 make_float2(a.p, b.p),     make_float2(a.H, b.H), make_float2(a.sr, b.sr),
                                 make_float2(a.mn, b.mn),   make_float2(a.mt, b.mt)};
     };
     float2 o[4];
-    roe_flux_rot<LaneF2>(pair(lx, ly), pair(rx, ry), make_float2(hx_face, hy_face), o);
+    roe_flux_rot<LaneF2>(pair(lx, ly), pair(rx, ry), make_float2(hx, hy), o);
     fx[0] = o[0].x;
     fx[1] = o[1].x;
     fx[2] = o[2].x;

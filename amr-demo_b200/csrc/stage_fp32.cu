@@ -106,21 +106,21 @@ const void *cfl_kernel_fp32(int n)
     StageLaunch{N, QPB, T, MINB, StageSmem<N, QPB, true>::total,                               \
                 (const void *)stage_kernel<N, QPB, T, MINB, true, FluxOpsFP32>}
 
-// row-sweep kernel for 16x16 patches: one warp per quad, "quads per
-// block" = warps per block, no dynamic shared memory; all at 128
-// registers (16 resident warps per SM): fewer registers spill and run slower
+// row-sweep kernel for 16x16 patches: one warp per quad, "quads per block" =
+// warps per block; all at 128 registers (16 resident warps per SM): fewer
+// registers spill and run slower
 #define AMRGPU_SWEEP16(W, MINB)                                                                          \
-    StageLaunch{16, W, 32 * (W), MINB, 0, (const void *)sweep16_kernel<W, MINB>, 1,                      \
+    StageLaunch{16, W, 32 * (W), MINB, SweepSmem::bytes(W), (const void *)sweep16_kernel<W, MINB>, 1,    \
                 {(const void *)sweep16_kernel<W, MINB, 1>, (const void *)sweep16_kernel<W, MINB, 2>,     \
                  (const void *)sweep16_kernel<W, MINB, 3>},                                               \
                 kSchemeRK3ShuOsher}
 #define AMRGPU_SWEEP8(W, MINB)                                                                           \
-    StageLaunch{8, 2 * (W), 32 * (W), MINB, 0, (const void *)sweep8_kernel<W, MINB>, 1,                  \
+    StageLaunch{8, 2 * (W), 32 * (W), MINB, SweepSmem::bytes(W), (const void *)sweep8_kernel<W, MINB>, 1,\
                 {(const void *)sweep8_kernel<W, MINB, 1>, (const void *)sweep8_kernel<W, MINB, 2>,       \
                  (const void *)sweep8_kernel<W, MINB, 3>},                                                \
                 kSchemeRK3ShuOsher}
 #define AMRGPU_SWEEPMIX(W, MINB)                                                                         \
-    StageLaunch{0, W, 32 * (W), MINB, 0, (const void *)sweep_mixed_kernel<W, MINB>, 1,                   \
+    StageLaunch{0, W, 32 * (W), MINB, SweepSmem::bytes(W), (const void *)sweep_mixed_kernel<W, MINB>, 1, \
                 {(const void *)sweep_mixed_kernel<W, MINB, 1>, (const void *)sweep_mixed_kernel<W, MINB, 2>, \
                  (const void *)sweep_mixed_kernel<W, MINB, 3>},                                            \
                 kSchemeRK3ShuOsher}
