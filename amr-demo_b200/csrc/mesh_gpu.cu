@@ -446,46 +446,42 @@ __global__ void rank_kernel(int nq, QuadDesc *out, const int *emits, const int *
 // launches and a read-back per pass. The phases are the kernels above, item
 // for item, so the leaves, descriptors and tables are the same.
 
-// Device-wide barrier of a cooperative launch: the last block to arrive
-// resets the count and advances the generation; the others wait for the
-// generation to move, at most kBarrierSpins polls. A wait that runs out
-// sets `abort` and every block leaves at its next barrier, so a fault in the
-// loop's logic ends the kernel with an error instead of hanging it.
+// Device-wide barrier of a cooperative launch: one counter that only grows
+// (the launch clears it). A block adds one and waits until the count has
+// reached `target`, all blocks' arrivals so far, at most kBarrierSpins polls.
+// A wait that runs out sets kBarrierAbort in the counter and every block
+// leaves at its next barrier, so a fault in the loop's logic ends the kernel
+// with an error instead of hanging it.
+//
+// The barriers are most of the loop at a few thousand leaves (six phases a
+// pass, each a few dependent loads a thread): a generation word beside the
+// count, reset by the last block, cost a load before and three operations
+// after the last arrival, and the abort word one more load per barrier (a
+// loop over 6811 leaves: 75 us; with this barrier 59 us, 29,138 leaves 96 and
+// 82 us).
 constexpr long long kBarrierSpins = 1ll << 22;
+constexpr unsigned kBarrierAbort = 1u << 31;
+constexpr unsigned kBarrierWindow = 1u << 29;  // above every launch's arrivals
 
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p)
-{
-    unsigned v;
-    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ bool grid_barrier(BalanceCtl *ctl)
+__device__ bool grid_barrier(BalanceCtl *ctl, unsigned &target)
 {
     __shared__ int s_ok;
+    target += gridDim.x;
     __syncthreads();
     if (threadIdx.x == 0) {
-        const unsigned gen = ld_acquire_u32(&ctl->bar_gen);
-        __threadfence();
-        const unsigned arrived = atomicAdd(&ctl->bar_count, 1u) + 1u;
-        int ok = 1;
-        if (arrived == gridDim.x) {
-            atomicExch(&ctl->bar_count, 0u);
-            __threadfence();
-            atomicAdd(&ctl->bar_gen, 1u);
-        } else {
-            long long spins = 0;
-            while (ld_acquire_u32(&ctl->bar_gen) == gen) {
-                if (++spins > kBarrierSpins) {
-                    ok = 0;
-                    atomicExch(&ctl->abort, 1);
-                    break;
-                }
-                __nanosleep(64);
+        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(&ctl->bar_count) : "memory");
+        int ok = 0;
+        for (long long spins = 0; spins <= kBarrierSpins; ++spins) {
+            unsigned v;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(&ctl->bar_count) : "memory");
+            if (v & kBarrierAbort) break;
+            if (v - target < kBarrierWindow) {
+                ok = 1;
+                break;
             }
+            if (spins == kBarrierSpins) atomicOr(&ctl->bar_count, kBarrierAbort);
         }
-        __threadfence();
-        s_ok = ok && *(volatile int *)&ctl->abort == 0;
+        s_ok = ok;
     }
     __syncthreads();
     return s_ok != 0;
@@ -496,7 +492,8 @@ __device__ bool grid_barrier(BalanceCtl *ctl)
 // contiguous run of it; block sums go through bsum and a barrier. Returns
 // false when a barrier gave up.
 template <typename Cnt>
-__device__ bool grid_scan(int n, Cnt cnt, int *pos, int *bsum, BalanceCtl *ctl)
+__device__ bool grid_scan(int n, Cnt cnt, int *pos, int *bsum, BalanceCtl *ctl,
+                          unsigned &bar)
 {
     __shared__ int s_warp[32];
     __shared__ int s_off, s_tot;
@@ -527,7 +524,7 @@ __device__ bool grid_scan(int n, Cnt cnt, int *pos, int *bsum, BalanceCtl *ctl)
     __syncthreads();
     const int texcl = incl - sum + (w > 0 ? s_warp[w - 1] : 0);
     if (threadIdx.x == 0) bsum[blockIdx.x] = s_warp[nw - 1];
-    if (!grid_barrier(ctl)) return false;
+    if (!grid_barrier(ctl, bar)) return false;
     // this block's offset and the total, from every block's sum
     int off = 0, tot = 0;
     for (int b = threadIdx.x; b < (int)gridDim.x; b += T) {
@@ -553,7 +550,7 @@ __device__ bool grid_scan(int n, Cnt cnt, int *pos, int *bsum, BalanceCtl *ctl)
         run += cnt(i);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) pos[n] = s_tot;
-    return grid_barrier(ctl);
+    return grid_barrier(ctl, bar);
 }
 
 // The adapt phase's decisions for one leaf, those of forest_adapt
@@ -638,6 +635,7 @@ __device__ __forceinline__ void adapt_write_item(const AdaptArgs &ad, const int4
 __global__ void __launch_bounds__(256) balance_loop_kernel(const BalanceLoopArgs a)
 {
     BalanceCtl *ctl = a.ctl;
+    unsigned bar = 0;  // arrivals at the barriers so far, all blocks
     const int gtid = blockIdx.x * blockDim.x + threadIdx.x, gstride = gridDim.x * blockDim.x;
     int nl = a.nl, live = a.live, passes = 0;
     bool ok = true, done = false, overflow = false, refined = false;
@@ -648,8 +646,8 @@ __global__ void __launch_bounds__(256) balance_loop_kernel(const BalanceLoopArgs
         const int4 *in = a.leaves[live];
         unsigned char *fs = a.flags;
         for (int i = gtid; i < nl; i += gstride) fs[i] = adapt_family_start(a.ad, in, nl, i) ? 1 : 0;
-        ok = grid_barrier(ctl);
-        if (ok) ok = grid_scan(nl, [&](int i) { return adapt_count(a.ad, in, fs, i); }, a.pos, a.bsum, ctl);
+        ok = grid_barrier(ctl, bar);
+        if (ok) ok = grid_scan(nl, [&](int i) { return adapt_count(a.ad, in, fs, i); }, a.pos, a.bsum, ctl, bar);
         if (ok) {
             adapt_total = __ldcg(a.pos + nl);
             if (adapt_total > a.cap) {
@@ -658,7 +656,7 @@ __global__ void __launch_bounds__(256) balance_loop_kernel(const BalanceLoopArgs
                 for (int i = gtid; i < nl; i += gstride)
                     adapt_write_item(a.ad, in, fs, a.pos, a.leaves[1 - live], a.orig[1 - live], a.dirty[1 - live],
                                      i);
-                ok = grid_barrier(ctl);
+                ok = grid_barrier(ctl, bar);
                 live = 1 - live;
                 nl = adapt_total;
                 adapted = adapt_total;
@@ -672,7 +670,7 @@ __global__ void __launch_bounds__(256) balance_loop_kernel(const BalanceLoopArgs
         F.nq = nl;
         unsigned char *flags = a.flags;
         for (int i = gtid; i <= nl; i += gstride) pass_prep_item(F, a.ntrees, a.tree_begin, flags, i);
-        if (!(ok = grid_barrier(ctl))) break;
+        if (!(ok = grid_barrier(ctl, bar))) break;
         if (ndirty >= 0) {
             // the leaves the previous pass created, listed by its refinement
             for (int t = gtid; t < 16 * ndirty; t += gstride)
@@ -680,8 +678,8 @@ __global__ void __launch_bounds__(256) balance_loop_kernel(const BalanceLoopArgs
         } else {
             for (long long t = gtid; t < 16ll * nl; t += gstride) balance_check_item(F, a.dirty[live], flags, t);
         }
-        if (!(ok = grid_barrier(ctl))) break;
-        if (!(ok = grid_scan(nl, [&](int i) { return __ldcg(flags + i) ? 4 : 1; }, a.pos, a.bsum, ctl))) break;
+        if (!(ok = grid_barrier(ctl, bar))) break;
+        if (!(ok = grid_scan(nl, [&](int i) { return __ldcg(flags + i) ? 4 : 1; }, a.pos, a.bsum, ctl, bar))) break;
         const int total = __ldcg(a.pos + nl);
         if (total == nl) {
             done = true;
@@ -701,7 +699,7 @@ __global__ void __launch_bounds__(256) balance_loop_kernel(const BalanceLoopArgs
                 for (int c = 0; c < 4; ++c) a.dirty_list[k + c] = at + c;
             }
         }
-        if (!(ok = grid_barrier(ctl))) break;
+        if (!(ok = grid_barrier(ctl, bar))) break;
         ndirty = 4 * ((total - nl) / 3);
         live = 1 - live;
         nl = total;
@@ -724,8 +722,8 @@ __global__ void __launch_bounds__(256) balance_loop_kernel(const BalanceLoopArgs
             }
         }
         for (int t = gtid; t < 4 * nl; t += gstride) sides_item(F, a.out, a.emits, a.emitter, a.status, t);
-        ok = grid_barrier(ctl);
-        if (ok) ok = grid_scan(4 * nl, [&](int t) { return __ldcg(a.emits + t); }, a.scan, a.bsum, ctl);
+        ok = grid_barrier(ctl, bar);
+        if (ok) ok = grid_scan(4 * nl, [&](int t) { return __ldcg(a.emits + t); }, a.scan, a.bsum, ctl, bar);
         if (ok) {
             for (int t = gtid; t < 4 * nl; t += gstride) a.out[t >> 2].side[t & 3].rank = __ldcg(a.scan + a.emitter[t]);
             if (gtid == 0) a.status[1] = nl > 0 ? __ldcg(a.scan + 4 * nl) : 0;
@@ -815,13 +813,15 @@ cudaError_t launch_build_quads(const ForestDev &F, QuadDesc *out, int *emits, in
 cudaError_t launch_balance_loop(const BalanceLoopArgs &a, int sms, cudaStream_t st)
 {
     // one block per SM at most (a cooperative launch needs every block
-    // resident), fewer for small forests: about 8 of the 16 checks per leaf
-    // per thread, since every block takes part in every barrier
+    // resident), fewer for small forests, where more arrivals at a barrier
+    // cost what shorter chains of checks gain: two of the 16 checks per leaf
+    // per thread (whole regrid, 691 leaves: 97 us, with eight checks 99 us;
+    // 6811 leaves: 123.5 us, with four 124.5, with eight 136 us)
     int occ = 0;
     cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, balance_loop_kernel, 256, 0);
     if (e != cudaSuccess) return e;
     if (occ < 1) return cudaErrorLaunchOutOfResources;
-    const long long want = (16ll * std::max(a.nl, 1) + 8 * 256 - 1) / (8 * 256);
+    const long long want = (16ll * std::max(a.nl, 1) + 2 * 256 - 1) / (2 * 256);
     const int grid = int(std::max(1ll, std::min<long long>(want, (long long)sms)));
     BalanceLoopArgs args = a;
     void *p[] = {&args};

@@ -56,8 +56,7 @@ cudaError_t launch_balance_refine(int nq, const int4 *in, const int *orig_in, co
 // buffer `live` with nl leaves and ends with ctl->live / ctl->nl.
 enum { kBalanceDone = 1, kBalanceOverflow = 2, kBalanceNoConverge = 3, kBalanceTimeout = 4 };
 struct BalanceCtl {
-    unsigned bar_count, bar_gen;  // the barrier
-    int abort;                    // set by a barrier wait that ran out
+    unsigned bar_count;           // the barrier's arrivals; its top bit is set by a wait that ran out
     int nl, live, passes, refined;
     int result;                   // kBalance*
     int adapted;                  // leaves after the adapt phase (0: no adapt ran or it overflowed)
