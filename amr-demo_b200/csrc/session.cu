@@ -1786,8 +1786,8 @@ int apply_regrid(amrgpu_session *s, int nq, int nface, long long mixed_cells = -
         ra.cfl.nquad = nq;
         ra.cfl.slot = p;
         ra.cfl.cfl = s->cfg.cfl;
-        const long long cells_new = (long long)nq * s->n * s->n;
-        const int g = int(std::max(1ll, std::min<long long>((cells_new + 255) / 256, (long long)s->sms * 16)));
+        const long long pairs = (long long)nq * s->n * s->n / 2;  // a thread takes two cells
+        const int g = int(std::max(1ll, std::min<long long>((pairs + 255) / 256, (long long)s->sms * 16)));
         void *args[] = {&ra};
         if (ok) ok = cuda_ok(cudaLaunchKernel(rcfl, dim3(g), dim3(256), args, 0, s->stream), "remap + CFL kernel");
         s->launches++;
