@@ -613,8 +613,7 @@ __global__ void __launch_bounds__(kWgradThreads, 2) mlp_wgrad_kernel(const Wgrad
 // 32 ring cells (one a lane). Bound by the latency of a quad's loads and of
 // its divisions and root, which one warp now does once for the quad: a block
 // of four warps and three barriers per quad took 27 us for 6802 quads of 8x8
-// (14 MB read), this takes
-// 12 us.
+// (14 MB read), this takes 12 us.
 constexpr int kFeatWarps = 4;
 
 template <int N>
