@@ -20,12 +20,17 @@ namespace amrgpu {
 // stage kernels waited on that chain (FP64 pipe 41-45% busy). The functions
 // below return the same bits from fused multiply-adds alone, for operands
 // whose ranges are checked once per cell:
-//   recip_rn     RN(1/b): the approximation, one cubic step (the result is
-//                within one last place), then y + y (1 - b y), which rounds
-//                correctly for every mantissa but all ones (P. Markstein,
-//                "Computation of elementary functions on the IBM RISC
-//                System/6000 processor", 1990); that one ends on the tie
-//                1/2, one last place too low, and is set
+//   recip_rn     RN(1/b): the approximation y0, two factors of Goldschmidt's
+//                product y0 (1 + e) (1 + e^2), e = 1 - b y0 (R. E. Goldschmidt,
+//                "Applications of division by convergence", MIT, 1964), then
+//                y + y (1 - b y), which rounds correctly for every mantissa
+//                but all ones (P. Markstein, "Computation of elementary
+//                functions on the IBM RISC System/6000 processor", 1990).
+//                Markstein's step wants a y within one last place: next to a
+//                rounding boundary the product is one of the two doubles
+//                around 1/b (its two roundings are half a place each, and the
+//                doubles beyond are one and a half away). All ones ends on
+//                the tie 1/2, one last place too low, and is set
 //   quotient_by  RN(a/b) from y = RN(1/b): q = RN(a y), then
 //                RN(q + y RN(a - b q)) (Markstein; N. Brisebarre,
 //                J.-M. Muller and S. K. Raina, "Accelerating correctly
@@ -37,9 +42,10 @@ namespace amrgpu {
 //                close to a rounding boundary only for mantissas with
 //                x = k^2 + k + c, |c| <= 4 (in last places), which are
 //                among those checked
-// Checked against CUDA's IEEE operations on 5 G random and near-boundary
-// operands, on every such mantissa with |c| <= 4000 and on the 64 mantissas
-// at each end of the binade: no bit differs.
+// test_gpu_fp64_ops.py calls the three and finds no bit different from IEEE
+// in 5 x 2^30 random operands, the 4096 mantissas at each end of the binade,
+// the roots' mantissas with |c| <= 4000 and 20,000 quotients within 2^-103 of
+// a boundary, out to both ends of the stated ranges.
 //
 // Ranges: a cell record is marked (sign bit of its sqrt(rho), see
 // cell_prims_fp64) unless rho and rho E lie in [2^-40, 2^40) and each
@@ -72,7 +78,9 @@ __device__ __forceinline__ double recip_rn(double b)
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
     double e = __fma_rn(-b, y, 1.0);
-    y = __fma_rn(y, __fma_rn(e, e, e), y);
+    y = __fma_rn(y, e, y);
+    e = e * e;
+    y = __fma_rn(y, e, y);
     e = __fma_rn(-b, y, 1.0);
     y = __fma_rn(y, e, y);
     const unsigned ones = (unsigned)__double2loint(b) & ((unsigned)__double2hiint(b) | 0xfff00000u);
@@ -94,7 +102,8 @@ __device__ __forceinline__ double sqrt_rn(double x)
     return __fma_rn(__fma_rn(-g, g, x), h, g);
 }
 
-// a / b from y = RN(1/b)
+// RN(a/b) from y = RN(1/b): a zero or |a| in [2^-850, 2^700], |b| in
+// [2^-250, 2^250], |a/b| in [2^-950, 2^950]
 __device__ __forceinline__ double quotient_by(double a, double b, double y)
 {
     const double q = a * y;
