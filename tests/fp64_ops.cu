@@ -106,3 +106,34 @@ extern "C" int fp64_random(int op, unsigned long long seed, long long n, int alo
     cudaFree(d);
     return (int)e;
 }
+
+namespace {
+
+__global__ void marked_kernel(const double *q, int *marked, int n)
+{
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= n) return;
+    double P[9];
+    cell_prims_fp64(q + 4 * k, P);
+    marked[k] = __double2hiint(P[8]) < 0;
+}
+
+}  // namespace
+
+// Whether the records of n states [n][4] are marked. 0 or a CUDA error.
+extern "C" int fp64_marked(const double *q, int *marked, int n)
+{
+    double *d = nullptr;
+    const size_t in = sizeof(double) * 4 * (size_t)n, out = sizeof(int) * (size_t)n;
+    cudaError_t e = cudaMalloc(&d, in + out);
+    if (e != cudaSuccess) return (int)e;
+    int *m = reinterpret_cast<int *>(d + 4 * (size_t)n);
+    e = cudaMemcpy(d, q, in, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        marked_kernel<<<(n + 255) / 256, 256>>>(d, m, n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(marked, m, out, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return (int)e;
+}

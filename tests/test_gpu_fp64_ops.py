@@ -19,7 +19,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 RECIP, ROOT, QUOTIENT = 0, 1, 2
 # the stated ranges, as exponents: recip_rn and sqrt_rn take operands in
 # [2^-500, 2^500]; quotient_by a zero or a numerator in [2^-850, 2^700] over a
-# divisor in [2^-250, 2^250], with the quotient in [2^-950, 2^950]
+# divisor in [2^-320, 2^320], with the quotient in [2^-950, 2^950]
 RANGE = 500
 
 
@@ -33,6 +33,7 @@ def ops(tmp_path_factory):
     L = C.CDLL(str(so))
     f64p = C.POINTER(C.c_double)
     L.fp64_ops.argtypes = [C.c_int, f64p, f64p, f64p, C.c_longlong]
+    L.fp64_marked.argtypes = [f64p, C.POINTER(C.c_int), C.c_int]
     L.fp64_random.argtypes = [C.c_int, C.c_ulonglong, C.c_longlong] + [C.c_int] * 4 + [C.POINTER(C.c_ulonglong)]
     return L
 
@@ -65,7 +66,7 @@ def test_roots_nearest_to_a_tie(ops):
 def test_quotients_nearest_to_a_tie(ops):
     a, b = X.near_tie_quotients(np.random.default_rng(0), 20000)
     # (numerator, divisor) exponents at the corners of the range
-    for ea, eb in ((0, 0), (699, 249), (699, -250), (-850, 100), (-850, -250), (-700, 249), (-700, -200), (512, -134)):
+    for ea, eb in ((0, 0), (699, 319), (699, -249), (-850, 99), (-850, -320), (-630, 319), (-700, -200), (512, -301)):
         for s in (1.0, -1.0):
             check(ops, QUOTIENT, s * a * 2.0 ** ea, b * 2.0 ** eb)
 
@@ -79,7 +80,7 @@ def test_quotients_by_binade_ends(ops):
 
 
 def test_zero_numerators(ops):
-    b = scaled(X.binade_ends(64), [-250, 0, 249])
+    b = scaled(X.binade_ends(64), [-320, 0, 319])
     check(ops, QUOTIENT, 0.0, np.concatenate([b, -b]))
     check(ops, QUOTIENT, -0.0, b)  # compares equal to a zero of either sign
 
@@ -87,8 +88,8 @@ def test_zero_numerators(ops):
 @pytest.mark.parametrize("op,a,b", [
     (RECIP, (0, 0), (-RANGE, RANGE - 1)),
     (ROOT, (0, 0), (-RANGE, RANGE - 1)),
-    (QUOTIENT, (-850, 699), (-250, 99)),
-    (QUOTIENT, (-700, 699), (-250, 249)),
+    (QUOTIENT, (-850, 628), (-320, 99)),
+    (QUOTIENT, (-629, 699), (-249, 319)),
     (QUOTIENT, (-60, 60), (-60, 60)),
 ])
 def test_random_operands(ops, op, a, b):
@@ -96,3 +97,32 @@ def test_random_operands(ops, op, a, b):
     bad = C.c_ulonglong(1)
     assert ops.fp64_random(op, 0x1234, 1 << 30, *a, *b, C.byref(bad)) == 0
     assert bad.value == 0
+
+
+@pytest.mark.parametrize("rho,speed", [(1.0, 1.0), (1e-24, 1e6), (1e-31, 1e9), (1.2, 340.0), (1.2e-3, 3.4e4),
+                                       (1e30, 1.0), (1.0, 1e-12)])
+def test_states_in_any_units_are_not_marked(ops, rho, speed):
+    """Densities and speeds of CGS, SI and scaled units, with one velocity
+    zero, tiny (ahead of a shock) or as large as the other."""
+    q = np.array([[rho, rho * speed * m, rho * speed * k, rho * speed ** 2 * 2.5]
+                  for m in (1.0, -0.3) for k in (0.0, -0.0, 1.0, 1e-30)])
+    marked = np.ones(len(q), np.int32)
+    assert ops.fp64_marked(q.ctypes.data_as(C.POINTER(C.c_double)), marked.ctypes.data_as(C.POINTER(C.c_int)),
+                           len(q)) == 0
+    assert not marked.any()
+
+
+def test_states_out_of_range_are_marked(ops):
+    t = 2.0 ** -52
+    bad = [[0.0, 0, 0, 1], [-1.0, 0, 0, 1], [np.nan, 0, 0, 1], [np.inf, 0, 0, 1], [1.0, 0, 0, 0], [1.0, 0, 0, -1.0],
+           [1.0, 0, 0, np.nan], [2.0 ** 110, 0, 0, 2.0 ** 110], [2.0 ** -110 * (1 - t), 0, 0, 2.0 ** -110],
+           [1.0, 0, 0, 2.0 ** 80], [1.0, 0, 0, 2.0 ** -80 * (1 - t)], [1.0, 2.0 ** 100, 0, 1], [1.0, 0, -2.0 ** 100, 1],
+           [1.0, 2.0 ** -160 * (1 - t), 0, 1], [1.0, 0, 2.0 ** -161, 1], [1.0, np.nan, 0, 1], [1.0, 0, np.inf, 1],
+           [2.0 ** 109, 5e-324, 0, 2.0 ** 109]]
+    good = [[2.0 ** 110 * (1 - t), 0, 0, 2.0 ** 110], [2.0 ** -110, 0, 0, 2.0 ** -110], [1.0, 0, 0, 2.0 ** 80 * (1 - t)],
+            [1.0, 0, 0, 2.0 ** -80], [1.0, 2.0 ** 99, -2.0 ** -160, 1]]
+    q = np.array(bad + good, float)
+    marked = np.full(len(q), -1, np.int32)
+    assert ops.fp64_marked(q.ctypes.data_as(C.POINTER(C.c_double)), marked.ctypes.data_as(C.POINTER(C.c_int)),
+                           len(q)) == 0
+    assert marked.tolist() == [1] * len(bad) + [0] * len(good)
