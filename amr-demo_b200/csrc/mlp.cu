@@ -1048,14 +1048,19 @@ bool MlpState::refresh_bf16()
     std::vector<bf> w1(size_t(kH1) * kFeatIn), w2(size_t(kH2) * kH1), w3(size_t(kOutPad) * kH2, zero),
         w2t(size_t(kH1) * kH2), w3t(size_t(kH2) * kOutPad, zero);
     std::vector<float> b3(kOutPad, 0.0f);
-    for (int k = 0; k < kH1 * kFeatIn; ++k)
-        w1[size_t(tiled_index(kH1, k / kFeatIn, k % kFeatIn))] = __float2bfloat16(h[size_t(kParamOff[0] + k)]);
+    // piece by piece of 8 in a row: element by element through tiled_index,
+    // two divisions and a scattered store each, it takes 200 us more (set_params
+    // 450 us, so 252 us)
+    auto pieces = [](const float *src, int rows, int cols, bf *dst) {
+        for (int c = 0; c < cols / 8; ++c)
+            for (int o = 0; o < rows; ++o)
+                for (int k = 0; k < 8; ++k)
+                    dst[tiled_index(rows, o, 8 * c) + k] = __float2bfloat16(src[o * cols + 8 * c + k]);
+    };
+    pieces(h.data() + kParamOff[0], kH1, kFeatIn, w1.data());
+    pieces(h.data() + kParamOff[2], kH2, kH1, w2.data());
     for (int o = 0; o < kH2; ++o)
-        for (int i = 0; i < kH1; ++i) {
-            const bf b = __float2bfloat16(h[size_t(kParamOff[2] + o * kH1 + i)]);
-            w2[size_t(tiled_index(kH2, o, i))] = b;
-            w2t[size_t(tiled_index(kH1, i, o))] = b;
-        }
+        for (int i = 0; i < kH1; ++i) w2t[size_t(tiled_index(kH1, i, o))] = w2[size_t(tiled_index(kH2, o, i))];
     for (int o = 0; o < kOut; ++o) {
         for (int i = 0; i < kH2; ++i) {
             const bf b = __float2bfloat16(h[size_t(kParamOff[4] + o * kH2 + i)]);
