@@ -7,10 +7,13 @@
 //   AMRGPU_TUNE_CACHE=<path>   the file (empty: memory only)
 //   default                    $XDG_CACHE_HOME/amrgpu/tune.json, else
 //                              $HOME/.cache/amrgpu/tune.json
-// The file is {"amrgpu_tune": 1, "entries": [ {...}, ... ]} with one entry
-// object per line; it is rewritten through a temporary file and a rename,
-// so a reader never sees a half-written file. Unreadable or malformed
-// lines are skipped.
+// The file is {"amrgpu_tune": 1, "kernels": K, "entries": [ {...}, ... ]}
+// with one entry object per line; it is rewritten through a temporary file
+// and a rename, so a reader never sees a half-written file. Unreadable or
+// malformed lines are skipped. K is the checksum of the stage kernels'
+// sources that this library was built from (the Makefile's TUNE_REVISION): a
+// file of other kernels, whose times and ranking are theirs, is not read and
+// is replaced by the first choice made.
 #include <sys/stat.h>
 #include <unistd.h>
 
@@ -23,6 +26,10 @@
 #include <vector>
 
 #include "amrgpu_internal.h"
+
+#ifndef AMRGPU_TUNE_REVISION
+#error "AMRGPU_TUNE_REVISION: the checksum of the stage kernels' sources (Makefile)"
+#endif
 
 namespace amrgpu {
 
@@ -52,7 +59,12 @@ void load_locked()
     FILE *fp = std::fopen(path.c_str(), "r");
     if (!fp) return;
     char line[512];
+    unsigned long kernels = 0;
+    bool ours = false;
     while (std::fgets(line, sizeof(line), fp)) {
+        if (std::sscanf(line, "{\"amrgpu_tune\": 1, \"kernels\": %lu,", &kernels) == 1)
+            ours = kernels == AMRGPU_TUNE_REVISION;
+        if (!ours) continue;
         const char *p = std::strstr(line, "{\"gpu\": \"");
         if (!p) continue;
         TuneEntry e;
@@ -79,7 +91,7 @@ void save_locked()
     const std::string tmp = path + ".tmp." + std::to_string((long)getpid());
     FILE *fp = std::fopen(tmp.c_str(), "w");
     if (!fp) return;  // read-only location: the choices stay in memory
-    std::fprintf(fp, "{\"amrgpu_tune\": 1, \"entries\": [\n");
+    std::fprintf(fp, "{\"amrgpu_tune\": 1, \"kernels\": %lu, \"entries\": [\n", AMRGPU_TUNE_REVISION);
     for (size_t k = 0; k < g_entries.size(); ++k) {
         const TuneEntry &e = g_entries[k];
         std::fprintf(fp,

@@ -262,8 +262,8 @@ int amrgpu_session_set_launch(amrgpu_session_t *s, int quads_per_block, int thre
  * stored per (GPU name, SM count, form, patch size, floor(log2(quads))) in
  * memory and in a JSON file -- AMRGPU_TUNE_CACHE (empty: memory only), else
  * $XDG_CACHE_HOME/amrgpu/tune.json or $HOME/.cache/amrgpu/tune.json -- and
- * later sessions with the same key use it without timing. hpc_amr_evolve_solver,
- * physics_go_gpu and every regrid go through the same path.
+ * later sessions with the same key use it without timing; a file written by a
+ * build of other stage kernels is not read. hpc_amr_evolve_solver, physics_go_gpu and every regrid go through the same path.
  * amrgpu_session_autotune tunes now (retime = 1: ignore the stored choice
  * and time again); the chosen shape is then amrgpu_session_launch_variant. */
 int amrgpu_session_autotune(amrgpu_session_t *s, int retime);

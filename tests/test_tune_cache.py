@@ -65,3 +65,21 @@ def test_empty_path_keeps_choices_in_memory(ag, cache_env, tmp_path):
     ag.lib().amrgpu_tune_cache_put(b"M", 148, 0, 16, 1024, 4, 128, 4, 0.1)
     assert _get(ag, "M", 0, 16, 1024) == (4, 128, 4, 0.1)
     assert not any(tmp_path.rglob("*.json"))
+
+
+@pytest.mark.parametrize("header", ['{"amrgpu_tune": 1, "entries": [', '{"amrgpu_tune": 1, "kernels": 1, "entries": ['],
+                         ids=["no revision", "another revision"])
+def test_choices_of_other_kernels_are_not_read(ag, cache_env, header):
+    """A file that another build of the stage kernels wrote: its entries are
+    as if absent, and the next choice replaces the file."""
+    L = ag.lib()
+    L.amrgpu_tune_cache_put(b"G", 148, 0, 16, 1024, 4, 128, 4, 0.3)
+    text = cache_env.read_text().splitlines()
+    ours = text[0]
+    cache_env.write_text("\n".join([header] + text[1:]) + "\n")
+    L.amrgpu_tune_cache_reload()
+    assert _get(ag, "G", 0, 16, 1024) is None
+    L.amrgpu_tune_cache_put(b"G", 148, 1, 8, 64, 1, 160, 2, 0.1)
+    assert cache_env.read_text().splitlines()[0] == ours
+    L.amrgpu_tune_cache_reload()
+    assert _get(ag, "G", 0, 16, 1024) is None and _get(ag, "G", 1, 8, 64) == (1, 160, 2, 0.1)
