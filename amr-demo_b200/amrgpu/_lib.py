@@ -83,6 +83,7 @@ PROTOTYPES = {
     "amrgpu_has_comm_ops": (C.c_int, []),
     "amrgpu_session_autotune": (C.c_int, [C.c_void_p, C.c_int]),
     "amrgpu_session_launch_variant_info": (C.c_int, [C.c_void_p, C.c_int, i32p, i32p, i32p, i32p]),
+    "amrgpu_default_launch": (C.c_int, [C.c_int, C.c_int, C.c_int, C.c_int, i32p, i32p, i32p]),
     "amrgpu_tune_cache_get": (C.c_int, [C.c_char_p, C.c_int, C.c_int, C.c_int, C.c_int, i32p, i32p, i32p, f64p]),
     "amrgpu_tune_cache_put": (C.c_int, [C.c_char_p, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int, C.c_int,
                                         C.c_double]),

@@ -23,9 +23,9 @@ struct StageLaunch {
     // RK3 of the FP64 form), when the variant has them
     const void *kernel_so[3] = {nullptr, nullptr, nullptr};
     int so_scheme = -1;
-    // a block kernel that is the default for meshes of at most this many
-    // quads (0: for none)
-    int small_quads = 0;
+    // 1: a block kernel that is the default for meshes small enough to be
+    // resident at once, quads <= qpb * min_blocks * SMs
+    int small = 0;
 };
 
 int stage_table_fp64(const StageLaunch **out);

@@ -483,8 +483,9 @@ bool quads_are_rectangles(const amrgpu_session *s)
 // pair, each running a serial sweep) gives way to the first block kernel
 // when the mesh has too few quads to occupy the GPU with sweep warps
 // (fewer than 1024 warps: measured slower on 256-1024 quads, faster from
-// 2048 warps on); the smallest meshes take the entry marked for them.
-const StageLaunch *default_launch(int form, int n, int nquad)
+// 2048 warps on); meshes whose quads are all resident at once in the entry
+// marked for small meshes take that one.
+const StageLaunch *default_launch(int form, int n, int nquad, int sms)
 {
     const StageLaunch *tab;
     const int cnt = (form == AMRGPU_FORM_FP32_FLUX) ? stage_table_fp32(&tab) : stage_table_fp64(&tab);
@@ -493,7 +494,7 @@ const StageLaunch *default_launch(int form, int n, int nquad)
         if (tab[i].n != n) continue;
         if (!first) first = &tab[i];
         if (!block && !tab[i].sweep) block = &tab[i];
-        if (!small && nquad <= tab[i].small_quads) small = &tab[i];
+        if (!small && tab[i].small && nquad <= tab[i].qpb * tab[i].min_blocks * sms) small = &tab[i];
     }
     if (small) return small;
     if (first && first->sweep && block) {
@@ -508,7 +509,7 @@ const StageLaunch *default_launch(int form, int n, int nquad)
 // default_launch.
 const StageLaunch *session_default_launch(const amrgpu_session *s)
 {
-    return s->mixed ? stage_launch_mixed() : default_launch(s->form, s->n, s->nquad);
+    return s->mixed ? stage_launch_mixed() : default_launch(s->form, s->n, s->nquad, s->sms);
 }
 
 const StageLaunch *find_launch(int form, int n, int qpb, int threads)
@@ -1037,7 +1038,7 @@ int amrgpu_session_set_form(amrgpu_session_t *s, int form)
     s->cfg.form = form;
     s->launch_pinned = false;
     s->tune_pending = true;
-    return configure_launch(s, default_launch(form, s->n, s->nquad));
+    return configure_launch(s, default_launch(form, s->n, s->nquad, s->sms));
 }
 
 int amrgpu_session_set_launch(amrgpu_session_t *s, int qpb, int threads)
@@ -1098,6 +1099,17 @@ int amrgpu_session_launch_variants(const amrgpu_session_t *s, int *qpb, int *thr
         ++k;
     }
     return k;
+}
+
+int amrgpu_default_launch(int form, int n, int nquad, int sms, int *qpb, int *threads, int *min_blocks)
+{
+    const bool known = form == AMRGPU_FORM_FP64_EXACT || form == AMRGPU_FORM_FP32_FLUX;
+    const StageLaunch *L = known && nquad >= 0 && sms > 0 ? default_launch(form, n, nquad, sms) : nullptr;
+    if (!L) return AMRGPU_ERR_ARG;
+    if (qpb) *qpb = L->qpb;
+    if (threads) *threads = L->threads;
+    if (min_blocks) *min_blocks = L->min_blocks;
+    return AMRGPU_OK;
 }
 
 int amrgpu_session_launch_variant_info(const amrgpu_session_t *s, int index, int *qpb, int *threads,

@@ -121,10 +121,10 @@ const void *cfl_kernel_fp64(int n)
     StageLaunch{N, QPB, T, MINB, StageSmem<N, QPB, false>::total,                              \
                 (const void *)stage_kernel<N, QPB, T, MINB, false, FluxOpsFP64>}
 
-// ... the default up to Q quads
-#define AMRGPU_STAGE64_SMALL(N, QPB, T, MINB, Q)                                                         \
+// ... the default for meshes that are resident at once
+#define AMRGPU_STAGE64_SMALL(N, QPB, T, MINB)                                                            \
     StageLaunch{N, QPB, T, MINB, StageSmem<N, QPB, false>::total,                                        \
-                (const void *)stage_kernel<N, QPB, T, MINB, false, FluxOpsFP64>, 0, {nullptr, nullptr, nullptr}, -1, Q}
+                (const void *)stage_kernel<N, QPB, T, MINB, false, FluxOpsFP64>, 0, {nullptr, nullptr, nullptr}, -1, 1}
 
 // row-sweep kernels: one warp per 16x16 quad or per two 8x8 quads
 #define AMRGPU_SWEEP64_16(W, MINB)                                                                      \
@@ -148,13 +148,14 @@ const void *cfl_kernel_fp64(int n)
 // 512 quads 11.7 -> 10.9 us (two rounds; the tuner's choice there is 96
 // threads at four blocks per SM, 8.3 us), 1024 quads 11.9 -> 18.3 us; 64
 // quads of 16x16 9.1 -> 8.0 us, 192 quads 10.3 -> 13.2 us. Hence the limits:
-// as many quads as blocks are resident, two per SM and one per SM.
+// as many quads as blocks are resident, two per SM and one per SM (296 and
+// 148 quads on 148 SMs).
 static const StageLaunch kTable64[] = {
     AMRGPU_SWEEP64_16(4, 3),  // 168 registers, 12 warps per SM
     AMRGPU_SWEEP64_16(4, 4),  // 128 registers, 16 warps per SM
     AMRGPU_SWEEP64_16(2, 8),
     AMRGPU_STAGE64(16, 1, 288, 2),
-    AMRGPU_STAGE64_SMALL(16, 1, 288, 1, 148),
+    AMRGPU_STAGE64_SMALL(16, 1, 288, 1),
     AMRGPU_STAGE64(16, 2, 576, 1),
     AMRGPU_STAGE64(16, 1, 256, 2),
     AMRGPU_SWEEP64_8(4, 3),   // two 8x8 quads per warp
@@ -162,7 +163,7 @@ static const StageLaunch kTable64[] = {
     AMRGPU_STAGE64(8, 4, 288, 2),
     AMRGPU_STAGE64(8, 2, 160, 3),
     AMRGPU_STAGE64(8, 4, 576, 1),
-    AMRGPU_STAGE64_SMALL(8, 1, 160, 2, 296),
+    AMRGPU_STAGE64_SMALL(8, 1, 160, 2),
     AMRGPU_STAGE64(8, 1, 96, 4),
     AMRGPU_STAGE64(4, 8, 160, 3),
     AMRGPU_STAGE64(4, 16, 320, 2),

@@ -263,7 +263,8 @@ int amrgpu_session_set_launch(amrgpu_session_t *s, int quads_per_block, int thre
  * memory and in a JSON file -- AMRGPU_TUNE_CACHE (empty: memory only), else
  * $XDG_CACHE_HOME/amrgpu/tune.json or $HOME/.cache/amrgpu/tune.json -- and
  * later sessions with the same key use it without timing; a file written by a
- * build of other stage kernels is not read. hpc_amr_evolve_solver, physics_go_gpu and every regrid go through the same path.
+ * build of other stage kernels is not read. hpc_amr_evolve_solver,
+ * physics_go_gpu and every regrid go through the same path.
  * amrgpu_session_autotune tunes now (retime = 1: ignore the stored choice
  * and time again); the chosen shape is then amrgpu_session_launch_variant. */
 int amrgpu_session_autotune(amrgpu_session_t *s, int retime);
@@ -276,6 +277,11 @@ int amrgpu_tune_cache_put(const char *gpu, int sms, int form, int n, int nquad, 
                           int threads, int min_blocks, double ms);
 /* Forgets the in-memory choices (the file is read again on next use). */
 void amrgpu_tune_cache_reload(void);
+
+/* The launch shape that a uniform mesh of nquad n x n quads has by default on
+ * a GPU of `sms` SMs (no GPU needed): the same choice a new session makes. */
+int amrgpu_default_launch(int form, int n, int nquad, int sms, int *quads_per_block, int *threads,
+                          int *min_blocks);
 
 /* The compiled stage-kernel launch shapes for the session's form and patch
  * size (the autotuner's candidates): fills up to cap pairs, returns the count. */
