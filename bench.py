@@ -22,7 +22,10 @@ fused stage kernels, the next step's CFL minimum folded into the last one).
 `--impl reference` times the reference's own CPU path (its C driver over
 the restated Fortran kernels, oracle/_ref, compiled -O3) on the same 1024^2
 mesh on all host cores instead: one MPI rank per core (threads over a
-multi-rank MPI stand-in, the reference's ghost exchange every stage).
+multi-rank MPI stand-in, the reference's ghost exchange every stage). Where
+oracle/_ref was not built (no reference tree), that arm says so in
+"unavailable", and the CPU baseline of both arms is the restatement of the
+reference's driver and kernels (oracle/_build) on one core, kind "port".
 """
 import argparse
 import json
@@ -86,6 +89,17 @@ def host_cores():
         return os.cpu_count() or 1
 
 
+def reference_missing():
+    """Why the reference's own CPU path cannot run here, or None."""
+    from oracle import oracle as O
+    for base in ("libref_physics_mt", "libref_physics"):
+        path = O.timing_build(base)[0]
+        if not os.path.exists(path):
+            return (f"oracle/_ref/{os.path.basename(path)} is not built: the reference's sources were not there when "
+                    "the oracle was made")
+    return None
+
+
 def cpu_baseline(steps=10, one_rank_steps=2, level=6):
     """The reference's own CPU path on this host, on the benchmark's own
     workload (the 1024^2 vortex mesh, built in NumPy by oracle/workload.py:
@@ -95,12 +109,25 @@ def cpu_baseline(steps=10, one_rank_steps=2, level=6):
     rank holding a Morton range of quads plus its ghost quads and
     exchanging them every stage as physics_mpi_real_to_ghost does. value =
     cells x steps / the slowest rank's time in physics_go. A one-rank run of
-    the same mesh is reported beside it."""
+    the same mesh is reported beside it. Without the reference's libraries:
+    the restatement alone, on one core."""
     from oracle import oracle as O, workload as WL
     from amrgpu import shard as S  # NumPy partitioning only; the library is not loaded
     n = 16
     mesh = WL.uniform_periodic_mesh(level, n)
     s0 = WL.vortex_state(mesh)
+    missing = reference_missing()
+    if missing:
+        q = s0.copy()
+        t0 = time.perf_counter()
+        O.evolve(mesh, q, O.make_config(n, WL.vortex_config(n, steps=steps)))
+        value = mesh.ncells * steps / (time.perf_counter() - t0)
+        return {"value": value, "unit": UNIT, "cores": 1, "kind": "port",
+                "sample": f"the restatement of the reference's driver and kernels (-O2 -ffp-contract=off) on the "
+                          f"{int(round(mesh.ncells ** 0.5))}^2 vortex mesh ({mesh.ncell} quads of 16x16), {steps} RK3 "
+                          f"steps on one core; {missing}",
+                "one_rank": {"value": value, "unit": UNIT, "cores": 1, "steps": steps, "sample": "the same run"},
+                "same_config": True}
     procs = max(1, min(host_cores(), 128, mesh.ncell))
     mt_path, flags = O.timing_build("libref_physics_mt")
     one_path, _ = O.timing_build("libref_physics")
@@ -773,7 +800,9 @@ def run_gpu(args):
 def run_reference(args):
     """The reference arm: the reference's own CPU path (cpu_baseline) on the
     benchmark's mesh, --warmup untimed steps then --steps timed steps on all
-    host cores; rank 0 of a torchrun launch alone runs it."""
+    host cores; rank 0 of a torchrun launch alone runs it. Without the
+    reference's libraries the line says why in "unavailable", and its figures
+    are the restatement's."""
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
         return
@@ -788,6 +817,10 @@ def run_reference(args):
             "config": {"workload": WORKLOAD, "parallelism": f"{cb['cores']} MPI ranks (threads) on host cores"},
             "cpu_baseline": cb,
             "e2e": {"value": value, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0}}
+    missing = reference_missing()
+    if missing:
+        line = {"impl": "reference", "unavailable": missing, **line}
+        line["config"]["parallelism"] = "the restatement on one host core"
     print(json.dumps(line), flush=True)
 
 
