@@ -2,9 +2,11 @@
 // operation. Included only by translation units built with -fmad=false, so
 // that no multiply-add is contracted and every result is the IEEE-rounded
 // value the reference's Fortran produces without FMA:
-//   roe_flux_fp64   flux_2d_module.F90:63-182 (flux_roe_2d)
-//   bc_flux_fp64    bc_2d_module.F90:14-75 + flux_2d_module.F90:13-60
-//   cfl_candidate   solver_time_step_2d_module.F90:106-116
+//   cell_prims_fp64, roe_flux_prim_fp64
+//                      flux_2d_module.F90:63-182 (flux_roe_2d)
+//   residual_rate      solver_residual_subgrid_2d_module.F90 (-R / volume)
+//   bc_flux_fp64       bc_2d_module.F90:14-75 + flux_2d_module.F90:13-60
+//   cfl_candidate_fp64 solver_time_step_2d_module.F90:106-116
 // gamma = 1.4 and gm1 = 0.4 are hard-coded exactly as there; the flux's
 // pressure uses (gamma - 1) = 0.3999999999999999, its sound speed 0.4.
 #pragma once
@@ -138,80 +140,6 @@ __device__ __forceinline__ void residual_rate(const double r[4], double vol, dou
     }
 }
 
-__device__ __forceinline__ void roe_flux_fp64(const double ql[4], const double qr[4],
-                                              double n0, double n1, double flux[4])
-{
-    const double gamma = 1.4;
-    const double gm1 = 0.4;
-    const double half = 0.5;
-    double mag = sqrt(n0 * n0 + n1 * n1);
-    double nx = n0 / mag;
-    double ny = n1 / mag;
-
-    double rhol = ql[0];
-    double oneOrhol = 1.0 / rhol;
-    double ul = ql[1] * oneOrhol;
-    double vl = ql[2] * oneOrhol;
-    double El = ql[3] * oneOrhol;
-    double pl = (gamma - 1.0) * (ql[3] - half * rhol * (ul * ul + vl * vl));
-    double Hl = El + pl * oneOrhol;
-    double unl = ul * nx + vl * ny;
-
-    double rhor = qr[0];
-    double oneOrhor = 1.0 / rhor;
-    double ur = qr[1] * oneOrhor;
-    double vr = qr[2] * oneOrhor;
-    double Er = qr[3] * oneOrhor;
-    double pr = (gamma - 1.0) * (qr[3] - half * rhor * (ur * ur + vr * vr));
-    double Hr = Er + pr * oneOrhor;
-    double unr = ur * nx + vr * ny;
-
-    double srl = sqrt(rhol);
-    double srr = sqrt(rhor);
-    double oneOroe_fact = 1.0 / (srl + srr);
-    double rhobar = sqrt(rhol * rhor);
-    double ubar = (ul * srl + ur * srr) * oneOroe_fact;
-    double vbar = (vl * srl + vr * srr) * oneOroe_fact;
-    double Hbar = (Hl * srl + Hr * srr) * oneOroe_fact;
-    double abar = sqrt(gm1 * (Hbar - half * (ubar * ubar + vbar * vbar)));
-    double unbar = ubar * nx + vbar * ny;
-    double Mnbar = unbar / abar;
-
-    double eigp = unbar + abar;
-    double eigm = unbar - abar;
-    double eigp_max = unr + abar;
-    double eigm_min = unl - abar;
-    double b1 = (eigp > 0.0 || eigp_max > 0.0) ? ((eigp > eigp_max) ? eigp : eigp_max) : 0.0;
-    double b2 = (eigm < 0.0 || eigm_min < 0.0) ? ((eigm < eigm_min) ? eigm : eigm_min) : 0.0;
-
-    double bcoeff = b1 * b2 / (b1 - b2);
-    double delta1 = (rhor - rhol) - (pr - pl) / (abar * abar);
-    double Mcoeff = 1.0 / (1.0 + fabs(Mnbar));
-    double bM = bcoeff * Mcoeff;
-    double db = b1 - b2;
-    double fluxl, fluxr, disp;
-
-    fluxl = ql[1] * nx + ql[2] * ny;
-    fluxr = qr[1] * nx + qr[2] * ny;
-    disp = bcoeff * (rhor - rhol) - bM * delta1;
-    flux[0] = ((b1 * fluxl - b2 * fluxr) / db + disp) * mag;
-
-    fluxl = (ql[1] * ul + pl) * nx + (ql[2] * ul) * ny;
-    fluxr = (qr[1] * ur + pr) * nx + (qr[2] * ur) * ny;
-    disp = bcoeff * (qr[1] - ql[1]) - bM * (delta1 * ubar + rhobar * (ur - ul - nx * (unr - unl)));
-    flux[1] = ((b1 * fluxl - b2 * fluxr) / db + disp) * mag;
-
-    fluxl = (ql[1] * vl) * nx + (ql[2] * vl + pl) * ny;
-    fluxr = (qr[1] * vr) * nx + (qr[2] * vr + pr) * ny;
-    disp = bcoeff * (qr[2] - ql[2]) - bM * (delta1 * vbar + rhobar * (vr - vl - ny * (unr - unl)));
-    flux[2] = ((b1 * fluxl - b2 * fluxr) / db + disp) * mag;
-
-    fluxl = (ql[3] + pl) * unl;
-    fluxr = (qr[3] + pr) * unr;
-    disp = bcoeff * (rhor * Hr - rhol * Hl) - bM * (delta1 * Hbar + rhobar * (Hr - Hl));
-    flux[3] = ((b1 * fluxl - b2 * fluxr) / db + disp) * mag;
-}
-
 // Per-cell primitive record shared by the four faces of a cell:
 // [0] rho [1] rho*u [2] rho*v [3] rho*E [4] u [5] v [6] p [7] H [8] sqrt(rho),
 // each computed by exactly the expression flux_roe_2d uses
@@ -322,11 +250,15 @@ __device__ __forceinline__ void roe_flux_ops(const double *L, const double *R, d
     flux[3] = (O::over(b1 * fluxl - b2 * fluxr, db, y) + disp) * mag;
 }
 
-// Any normal and any states: called, not inlined (marked states are rare,
-// so are normals off the axes in meshes of powers of two, and one copy per
-// call site would crowd the instruction cache). Records and flux in (x, y)
-// components; by value: as scalars they cost the callers 20-60 bytes more
-// spills a thread.
+// Any normal and any states: called, not inlined (one copy per call site
+// would crowd the instruction cache and spill). On a domain whose width and
+// corner are powers of two or whole numbers no interior normal is off its
+// axis; on any other (width 0.7, corner 0.1) rounding of the nodes tilts a
+// quarter to a third of them, so that nearly every row has one and its warp
+// comes here: 1024^2 RK3 takes 312 us per step there against 249 us (380 and
+// 356 us with every division and root IEEE's own). Records and flux in
+// (x, y) components; by value: as scalars they cost the callers 20-60 bytes
+// more spills a thread.
 struct Flux4 {
     double v[4];
 };

@@ -53,7 +53,8 @@ struct MlpState {
 
     // per-batch work buffers: features, labels, logits and classes (capacity
     // cap_batch rows), and for training (cap_train rows) the layers' outputs
-    // and gradients, row-major, and the weight-gradient partials
+    // and gradients, in 8-row core matrices (blocked_index in mlp.cu), and the
+    // weight-gradient partials
     int cap_batch = 0, cap_train = 0;
     __nv_bfloat16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *dL = nullptr, *dZ2 = nullptr, *dZ1 = nullptr;
     float *Lg = nullptr, *P1 = nullptr, *P2 = nullptr, *P3 = nullptr, *gb = nullptr, *gflat = nullptr;

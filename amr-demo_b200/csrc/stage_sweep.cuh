@@ -42,8 +42,10 @@
 // shared memory, 275 us with 107 KB); in two slots (109 KB) 251 us; with the
 // two edge rounds in one packed evaluation, their fluxes kept in FP32 and the
 // next item's descriptors fetched during the last row 241 us, and 83.4 ->
-// 71.3 us at 1024^2, 87.7 -> 77.8 us at 1024^2 in 8x8 patches. 20 warps per
-// SM at 96 registers were 28% slower (215 KB of shared memory).
+// 71.3 us at 1024^2, 87.7 -> 77.8 us at 1024^2 in 8x8 patches (one session
+// alone; with three sessions' streams overlapping 71 -> 64 us per step at
+// 1024^2 and 268 -> 247 us at 2048^2). 20 warps per SM at 96 registers were
+// 28% slower (215 KB of shared memory).
 #pragma once
 
 #include <type_traits>

@@ -41,10 +41,11 @@
 //
 // Bound by the FP64 pipe's latency at 12 warps per SM (168 registers, no
 // spills; 128 registers and 16 warps spill 84-212 bytes a thread and are 3%
-// slower). 1024^2 cells in 16x16 patches, RK3, one session alone: 357 us per
-// step with IEEE division and square root inline, 250 us with this file's
+// slower). 1024^2 cells in 16x16 patches, RK3, one session alone: 356 us per
+// step with IEEE division and square root inline, 249 us with this file's
 // arithmetic (flux_fp64.cuh) and order; with three sessions' streams
-// overlapping 309 -> 186 us per step.
+// overlapping 309 -> 187 us per step. That is for domains on which every
+// interior normal lies along its axis (roe_flux_any); elsewhere 380 -> 312 us.
 #pragma once
 
 #include "async_copy.cuh"
@@ -155,7 +156,7 @@ __device__ __forceinline__ void sweep64_body(const StageArgs &a)
             }
         }
         __syncwarp();
-        // the nodes of column 0 (lane l computes row l; the last row lane 0)
+        // the nodes of column 0 (lanes 0..N of a quad's 2N: lane l row l)
         if (l <= N) bilinear_node(g, -1.0, scale_factor * (double)l - 1.0, c0[2 * l], c0[2 * l + 1]);
 
         // ---------------- edges: round 0 sides 0 / 1, round 1 sides 2 / 3

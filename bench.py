@@ -781,7 +781,7 @@ def run_gpu(args):
             "plain_fp64": {"value": out[0]["value"], "ms_per_step": out[0]["ms_per_step"],
                            "achieved_gbs": out[0]["achieved_gbs"], "frac": out[0]["achieved_gbs"] / hbm,
                            "bytes_per_cell_update": B_ALG[0], "launch": out[0]["tune"],
-                           "bound": "fp64 pipe (IEEE div/sqrt sequences)"},
+                           "bound": "fp64 pipe latency"},
             "fp32_flux": {"value": out[1]["value"], "ms_per_step": out[1]["ms_per_step"]},
             "speedup_fp32_over_fp64": out[1]["value"] / out[0]["value"],
             "l1_rho_rel_fp32_vs_fp64": l1,
