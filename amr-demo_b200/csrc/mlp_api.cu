@@ -222,11 +222,16 @@ int amrgpu_mlp_train_epoch(amrgpu_mlp_t *m, const int *perm, long long n, int ba
 {
     if (!m || !perm || n < 0 || batch < 128 || batch % 128 != 0 || n > m->st.n_data) return AMRGPU_ERR_ARG;
     MlpState &ms = m->st;
-    for (long long k = 0; k < n; ++k)
-        if (perm[k] < 0 || perm[k] >= ms.n_data) {
-            set_error(AMRGPU_ERR_ARG, "train: permutation entry out of range");
-            return AMRGPU_ERR_ARG;
-        }
+    // (without a branch per entry: with one, the loop's speed depended on
+    // where the linker put it; a call of 65,535 rows and no whole batch took
+    // 70 us in one build and 79 us in another, and takes 51 us)
+    const unsigned rows_end = (unsigned)std::min<long long>(ms.n_data, 1ll << 31);
+    unsigned bad = 0;
+    for (long long k = 0; k < n; ++k) bad |= (unsigned)((unsigned)perm[k] >= rows_end);
+    if (bad) {
+        set_error(AMRGPU_ERR_ARG, "train: permutation entry out of range");
+        return AMRGPU_ERR_ARG;
+    }
     const long long nb = n / batch;
     // per 32 rows: a loss sum and the correct predictions; the wait flags of
     // the tensor-core kernels come back behind them

@@ -77,3 +77,28 @@ def test_judge_counts(ag, L, n, level, fraction):
         assert j["coarser"] == (((p == L.REFINE) & (t != L.REFINE)) | ((t == L.COARSEN) & (p != L.COARSEN))).sum()
     m.close()
     s.close()
+
+
+@pytest.mark.parametrize("at", [0, 100, 299])
+@pytest.mark.parametrize("entry", [-1, -2 ** 31, "rows", 2 ** 31 - 1])
+def test_permutation_entries_out_of_range_are_refused(ag, L, at, entry):
+    """Before anything is trained: the parameters stay as they were. Entry
+    299 is in no whole batch and is refused as well."""
+    f = meshes.uniform(8, 3, periodic=(1, 1))
+    s = ag.Session(f.mesh(8), meshes.make_config(8).apply(), form=1)
+    s.upload(f.initialize(8))
+    m = L.Mlp(seed=2)
+    while m.size() < 300:
+        m.append(s, 0.02)
+    before = m.get_params()
+    perm = np.arange(300, dtype=np.int32)
+    m.train_epoch(perm[:0], batch=128)
+    perm[at] = m.size() if entry == "rows" else entry
+    with pytest.raises(ag.AmrGpuError):
+        m.train_epoch(perm, batch=128)
+    assert np.array_equal(m.get_params(), before)
+    perm[at] = m.size() - 1
+    m.train_epoch(perm, batch=128)
+    assert not np.array_equal(m.get_params(), before)
+    m.close()
+    s.close()
